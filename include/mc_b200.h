@@ -323,6 +323,12 @@ int mc_resample_scatter(const mc_desc* d, const void* x, const void* map, const 
  * src/util/cuda/knn_layer.cu:13-32.  Limits: 1 <= k <= 32, k <= M, D <= 16. */
 int mc_knn(const float* ref, const float* query, int32_t B, int32_t D, int32_t M, int32_t N,
            int32_t k, int64_t* idx, float* dist, void* stream);
+/* The same with scratch memory: for D <= 3 and enough pairs the neighbours are searched among sorted
+ * leaves of references instead of all of them - identical results.  mc_knn_workspace_bytes is 0 where
+ * mc_knn is the better choice (ws == NULL calls it). */
+size_t mc_knn_workspace_bytes(int32_t B, int32_t D, int32_t M, int32_t N, int32_t k);
+int mc_knn_ws(const float* ref, const float* query, int32_t B, int32_t D, int32_t M, int32_t N,
+              int32_t k, int64_t* idx, float* dist, void* ws, size_t ws_bytes, void* stream);
 
 /* ---- point location on the icosphere hierarchy ------------------------------------------------
  * samples (n, 2) float (lon, lat) radians.  Levels 0..order of the mesh hierarchy are given as host

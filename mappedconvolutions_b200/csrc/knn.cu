@@ -1,13 +1,18 @@
-// Brute-force k nearest neighbours without the N x M distance matrix.
-//
-// Each thread owns one query point and a sorted top-k list held in registers; reference points
-// stream through shared memory in tiles that every thread of the block reads as a broadcast.
+// k nearest neighbours without the N x M distance matrix, three ways (the choice is at the bottom):
+//   * many queries, few pairs: one thread per query and a sorted top-k list in registers; reference
+//     points stream through shared memory in tiles that every thread of the block reads as a broadcast;
+//   * few queries: one or several warps per query, merged at the end;
+//   * many pairs, D <= 3: references and queries sorted along a Morton curve, 32 references to a leaf
+//     with its bounding box, and a warp of 32 neighbouring queries that only looks at leaves whose
+//     box can still hold one of the k nearest points.
 // Semantics restated from the reference's include/util/cuda/knn.cuh:
 //   distance  :82-103   ssd over the dimensions in order, here pinned to s = fmaf(t, t, s) with
 //                       t = ref_i - query_i starting from s = 0
 //   selection :125-189  stable insertion, strict '<'  ==  order by (distance, index)
 //   indices   :141,160,184  1-based
 //   sqrt      :199-205
+#include <cub/device/device_radix_sort.cuh>
+
 #include "common.cuh"
 
 namespace mc {
@@ -34,6 +39,68 @@ struct TopK {
   }
 };
 
+// The k <= 32 best of ONE query, spread over a warp: lane t holds the t-th best, ordered by (distance,
+// index).  Empty slots are (infinity, 0): nothing at an infinite distance (or NaN) ever enters, as in
+// TopK, and such a slot is written as index 0 (= -1 + 1).  A candidate costs about twenty instructions of
+// the whole warp and no branch that depends on the lane; a list per lane costs ten times that and is
+// walked by the lanes at different times.
+struct WarpTopK {
+  float d;    // this lane's entry
+  int i;
+  float thr;  // distance of entry k - 1: candidates beyond it cannot enter (warp uniform)
+
+  static __device__ __forceinline__ bool less(float da, int ia, float db, int ib) {
+    return da < db || (da == db && ia < ib);
+  }
+  __device__ __forceinline__ void init() { d = INFINITY; i = 0; thr = INFINITY; }
+  // first 32 candidates, one per lane: sorted at once
+  __device__ __forceinline__ void fill(float s, int j, int k, int lane) {
+    const bool ok = s < INFINITY;
+    d = ok ? s : INFINITY;
+    i = ok ? j : 0;
+#pragma unroll
+    for (int size = 2; size <= 32; size *= 2) {
+#pragma unroll
+      for (int o = size / 2; o > 0; o /= 2) {
+        const float od = __shfl_xor_sync(0xffffffffu, d, o);
+        const int oi = __shfl_xor_sync(0xffffffffu, i, o);
+        const bool low = ((lane & o) == 0) == ((lane & size) == 0);  // this lane keeps the smaller one
+        if (less(od, oi, d, i) == low) { d = od; i = oi; }
+      }
+    }
+    thr = __shfl_sync(0xffffffffu, d, k - 1);
+  }
+  // one candidate per lane; those within thr enter one after another.  IN_ORDER: candidates come in index
+  // order, so that one at distance thr cannot displace anything.
+  template <bool IN_ORDER>
+  __device__ __forceinline__ void offer(float s, int j, int k, int lane) {
+    unsigned m = __ballot_sync(0xffffffffu, IN_ORDER ? s < thr : s <= thr && s < INFINITY);
+    while (m) {
+      const int src = __ffs(m) - 1;
+      m &= m - 1;
+      const float cs = __shfl_sync(0xffffffffu, s, src);
+      const int cj = __shfl_sync(0xffffffffu, j, src);
+      if (IN_ORDER ? cs >= thr : cs > thr) continue;
+      const float ud = __shfl_up_sync(0xffffffffu, d, 1);
+      const int ui = __shfl_up_sync(0xffffffffu, i, 1);
+      if (less(cs, cj, d, i)) {
+        const bool above = lane > 0 && less(cs, cj, ud, ui);
+        d = above ? ud : cs;
+        i = above ? ui : cj;
+      }
+      thr = __shfl_sync(0xffffffffu, d, k - 1);
+    }
+  }
+};
+
+// Launched behind the search among sorted leaves, the all-pairs kernels only run if that has given up:
+// `crowded` counts the leaves in crowded places, see knn_leaves_kernel.
+struct KnnGate {
+  const int* crowded;  // null: run
+  int nleaf;           // leaves in all
+  __device__ __forceinline__ bool tree() const { return crowded && __ldg(crowded) <= nleaf / 8; }
+};
+
 constexpr int KNN_THREADS = 256;
 constexpr int KNN_TILE = 512;
 constexpr int KNN_DMAX = 16;
@@ -44,7 +111,8 @@ __global__ void __launch_bounds__(KNN_THREADS) knn_kernel(const float* __restric
                                                           const float* __restrict__ query, int D,
                                                           int M, int N, int k,
                                                           int64_t* __restrict__ idx,
-                                                          float* __restrict__ dist) {
+                                                          float* __restrict__ dist, KnnGate gate) {
+  if (gate.tree()) return;
   constexpr int DS = DT > 0 ? DT : KNN_DMAX;
   __shared__ float tile[DS][KNN_TILE];
   const int b = blockIdx.y;
@@ -90,10 +158,6 @@ __global__ void __launch_bounds__(KNN_THREADS) knn_kernel(const float* __restric
   }
 }
 
-template <int DT>
-static void knn_launch_big_k(const float* ref, const float* query, int B, int M, int N, int k,
-                             int64_t* idx, float* dist, cudaStream_t st);
-
 // D <= 4: reference points are staged per coordinate and visited two at a time with packed
 // fp32 arithmetic (fma.rn.f32x2): difference and square-accumulate of a PAIR of references cost
 // one instruction each per dimension.  Every lane of a packed operation is the same correctly
@@ -120,7 +184,8 @@ __global__ void __launch_bounds__(KNN2_THREADS, KMAX <= 12 ? KNN2_BLOCKS_PER_SM 
                                                                    const float* __restrict__ query,
                                                                    int M, int N, int k,
                                                                    int64_t* __restrict__ idx,
-                                                                   float* __restrict__ dist) {
+                                                                   float* __restrict__ dist, KnnGate gate) {
+  if (gate.tree()) return;
   __shared__ __align__(16) float tile[DT][KNN2_TILE];
   const int b = blockIdx.y;
   const float* rb = ref + (long)b * DT * M;
@@ -178,48 +243,515 @@ __global__ void __launch_bounds__(KNN2_THREADS, KMAX <= 12 ? KNN2_BLOCKS_PER_SM 
   }
 }
 
-template <int DT>
-static void knn_small_d_launch(const float* ref, const float* query, int B, int M, int N, int k,
-                               int64_t* idx, float* dist, cudaStream_t st) {
-  dim3 grid((unsigned)((N + KNN2_THREADS - 1) / KNN2_THREADS), (unsigned)B);
-  if (k <= 8) knn_small_d_kernel<DT, 8><<<grid, KNN2_THREADS, 0, st>>>(ref, query, M, N, k, idx, dist), MC_COUNT(1);
-  else if (k <= 12) knn_small_d_kernel<DT, 12><<<grid, KNN2_THREADS, 0, st>>>(ref, query, M, N, k, idx, dist), MC_COUNT(1);
-  else if (k <= 16) knn_small_d_kernel<DT, 16><<<grid, KNN2_THREADS, 0, st>>>(ref, query, M, N, k, idx, dist), MC_COUNT(1);
-  else knn_launch_big_k<DT>(ref, query, B, M, N, k, idx, dist, st);
+
+// ---- few queries: a warp, or several, per query -----------------------------------------------------
+// One thread per query leaves the chip idle when there are few: 200 queries are two blocks of the kernel
+// above, whose threads walk 160 000 references one after another (2.9 ms).  Here the lanes of a warp look
+// at 32 references at a time (coalesced loads, four in flight per coordinate) for one query, whose list is
+// spread over the lanes; wpq warps share a query's references and the first one merges their lists.
+constexpr int KNNW_WARPS = 8;       // warps of a block that takes several queries
+constexpr int KNNW_MAX_WARPS = 32;  // warps that share one query at most
+
+__device__ __forceinline__ void knn_store(int64_t* idx, float* dist, long o, float d, int i) {
+  idx[o] = d == INFINITY ? 0 : (int64_t)i + 1;
+  dist[o] = __fsqrt_rn(d);
 }
 
 template <int DT>
-static void knn_launch_k(const float* ref, const float* query, int B, int D, int M, int N, int k,
-                         int64_t* idx, float* dist, cudaStream_t st) {
+__global__ void __launch_bounds__(KNNW_MAX_WARPS * 32) knn_wide_kernel(const float* __restrict__ ref,
+                                                                   const float* __restrict__ query, int D,
+                                                                   int M, int N, int k, int wpq,
+                                                                   int64_t* __restrict__ idx,
+                                                                   float* __restrict__ dist, KnnGate gate) {
+  if (gate.tree()) return;
+  constexpr int DS = DT > 0 ? DT : KNN_DMAX;
+  __shared__ float sd[KNNW_MAX_WARPS][32];
+  __shared__ int si[KNNW_MAX_WARPS][32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int b = blockIdx.y;
+  const int n = blockIdx.x * (blockDim.x / 32 / wpq) + warp / wpq, part = warp % wpq;
+  const float* rb = ref + (long)b * D * M;
+  const float* qb = query + (long)b * D * N;
+  WarpTopK top;
+  top.init();
+  if (n < N) {
+    float q[DS];
+#pragma unroll
+    for (int i = 0; i < DS; ++i) q[i] = i < D ? __ldg(qb + (long)i * N + n) : 0.f;
+    constexpr int U = 4;
+    bool first = true;
+    for (int m0 = part * 32; m0 < M; m0 += wpq * 32 * U) {
+      float s[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) s[u] = 0.f;
+#pragma unroll
+      for (int i = 0; i < DS; ++i) {
+        if (DT == 0 && i >= D) break;
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          const int j = m0 + u * wpq * 32 + lane;
+          const float t = (j < M ? __ldg(rb + (long)i * M + j) : INFINITY) - q[i];
+          s[u] = fmaf(t, t, s[u]);
+        }
+      }
+      int u0 = 0;
+      if (first) { top.fill(s[0], m0 + lane, k, lane); first = false; u0 = 1; }
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (u >= u0) top.offer<true>(s[u], m0 + u * wpq * 32 + lane, k, lane);
+    }
+  }
+  if (wpq > 1) {
+    sd[warp][lane] = top.d;
+    si[warp][lane] = top.i;
+    __syncthreads();
+    if (part == 0)
+      for (int p = 1; p < wpq; ++p)
+        top.offer<false>(lane < k ? sd[warp + p][lane] : INFINITY, si[warp + p][lane], k, lane);
+  }
+  if (part == 0 && n < N && lane < k) knn_store(idx, dist, ((long)b * k + lane) * N + n, top.d, top.i);
+}
+
+// ---- many pairs: leaves on a Morton curve -----------------------------------------------------------
+// 163 842 x 163 842 points are 2.7e10 pairs: 7.6 ms at the rate of the packed arithmetic above, while
+// all but about a hundred references per query can be ruled out by their position.  Keys of all
+// references and queries (segment, 24-bit Morton code inside the bounding box of the references) are
+// radix sorted; 32 consecutive references of the order form a leaf, 32 leaves a node, 32 nodes a
+// group, each with the bounding box of its points.  A warp takes one query at a time: it starts with the
+// leaf where the query stands in the order (sorted at once), then its lanes test 32 boxes at a time and
+// the warp visits - one reference per lane - the leaves whose box is not farther from the query than its
+// k-th distance so far.  Consecutive warps take consecutive queries of the order, so that they meet the
+// same leaves in L1.
+// The box distance is formed like the point distance, with the gap to the box in place of the
+// coordinate difference: rounding is monotone, so it is never above the computed distance of any point
+// in the box, and "skip if box distance > k-th distance" cannot lose a point, ties included (equal
+// distances are ordered by index, hence no skip at equality).
+// NaN references are outside every box and never nearer than anything.
+// (Tried first: one query per lane and 32 neighbouring queries per warp, every lane testing the points of
+// all leaves that one of them needs: 271 us for the search alone, and far slower than all pairs where
+// queries are sparse among the references.)
+constexpr int KNNT_LEAF = 32;
+constexpr int KNNT_WARPS = 4;
+constexpr int KNNT_BITS = 24;
+
+__device__ __forceinline__ unsigned float_order(float f) {  // unsigned order == float order
+  const unsigned u = __float_as_uint(f);
+  return (u >> 31) ? ~u : u | 0x80000000u;
+}
+__device__ __forceinline__ float float_unorder(unsigned u) {
+  return __uint_as_float((u >> 31) ? u & 0x7fffffffu : ~u);
+}
+
+// bounds[b][0][i] = max of ~order(x) (i.e. the minimum), bounds[b][1][i] = max of order(x); zeroed before
+template <int DT>
+__global__ void __launch_bounds__(256) knn_bounds_kernel(const float* __restrict__ ref, int M,
+                                                         unsigned* __restrict__ bounds) {
+  const int b = blockIdx.y;
+  unsigned lo[DT], hi[DT];
+#pragma unroll
+  for (int i = 0; i < DT; ++i) lo[i] = hi[i] = 0u;
+  for (int j = blockIdx.x * 256 + threadIdx.x; j < M; j += gridDim.x * 256) {
+#pragma unroll
+    for (int i = 0; i < DT; ++i) {
+      const float v = __ldg(ref + ((long)b * DT + i) * M + j);
+      if (fabsf(v) <= FLT_MAX) {  // (no NaN, no infinity)
+        const unsigned o = float_order(v);
+        lo[i] = max(lo[i], ~o);
+        hi[i] = max(hi[i], o);
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < DT; ++i) {
+    lo[i] = __reduce_max_sync(0xffffffffu, lo[i]);
+    hi[i] = __reduce_max_sync(0xffffffffu, hi[i]);
+    if ((threadIdx.x & 31) == 0) {
+      atomicMax(bounds + ((long)b * 2 + 0) * DT + i, lo[i]);
+      atomicMax(bounds + ((long)b * 2 + 1) * DT + i, hi[i]);
+    }
+  }
+}
+
+template <int DT>
+__device__ __forceinline__ unsigned morton_spread(unsigned v) {
+  if (DT == 1) return v;
+  if (DT == 2) {
+    v = (v | (v << 8)) & 0x00FF00FFu; v = (v | (v << 4)) & 0x0F0F0F0Fu;
+    v = (v | (v << 2)) & 0x33333333u; return (v | (v << 1)) & 0x55555555u;
+  }
+  v = (v | (v << 16)) & 0x030000FFu; v = (v | (v << 8)) & 0x0300F00Fu;
+  v = (v | (v << 4)) & 0x030C30C3u;
+  return (v | (v << 2)) & 0x09249249u;
+}
+
+// key = segment << 24 | code; segments 0 .. B-1 are the references, B .. 2 B - 1 the queries
+template <int DT>
+__global__ void __launch_bounds__(256) knn_keys_kernel(const float* __restrict__ ref,
+                                                       const float* __restrict__ query, int B, int M, int N,
+                                                       const unsigned* __restrict__ bounds,
+                                                       unsigned* __restrict__ keys, int* __restrict__ vals) {
+  constexpr int BITS = KNNT_BITS / DT;
+  const long nref = (long)B * M, total = nref + (long)B * N;
+  for (long t = blockIdx.x * 256L + threadIdx.x; t < total; t += gridDim.x * 256L) {
+    const bool isq = t >= nref;
+    const long r = isq ? t - nref : t;
+    const int n = isq ? N : M;
+    const int b = (int)(r / n), j = (int)(r - (long)b * n);
+    unsigned code = 0;
+#pragma unroll
+    for (int i = 0; i < DT; ++i) {
+      const float v = __ldg((isq ? query : ref) + ((long)b * DT + i) * n + j);
+      const float lo = float_unorder(~__ldg(bounds + ((long)b * 2 + 0) * DT + i));
+      const float hi = float_unorder(__ldg(bounds + ((long)b * 2 + 1) * DT + i));
+      float f = (v - lo) * ((float)(1 << BITS) / fmaxf(hi - lo, 1e-37f));
+      f = fminf(fmaxf(f, 0.f), (float)((1 << BITS) - 1));  // (NaN becomes 0)
+      code |= morton_spread<DT>((unsigned)f) << i;
+    }
+    keys[t] = (unsigned)(isq ? B + b : b) << KNNT_BITS | code;
+    vals[t] = j;
+  }
+}
+
+// Leaf l of batch b: coordinates [DT][32] and original indices [32].  Boxes are stored 32 siblings
+// together, component by component - [parent][lo 0 .. lo DT-1, hi 0 .. hi DT-1][32] - so that a warp
+// reads each component of 32 boxes in one run (as structs they cost six times the L1 wavefronts, which
+// was half of the search's time); missing siblings are empty boxes, at infinite distance.
+// One warp per leaf, one block of 32 warps per node.
+// A curve of 8 bits per dimension cannot tell the points of one cell apart: a leaf whose cell fills 64
+// leaves and more is counted as crowded, and with more than an eighth of such leaves (points that nearly
+// all sit in one spot) the all-pairs kernels do the work instead.
+template <int DT>
+__global__ void __launch_bounds__(1024) knn_leaves_kernel(const float* __restrict__ ref, int M, int nleaf,
+                                                          const unsigned* __restrict__ keys,
+                                                          const int* __restrict__ vals, float* __restrict__ leaves,
+                                                          float* __restrict__ lbox, float* __restrict__ nbox,
+                                                          int ngroup, int* __restrict__ crowded) {
+  __shared__ float sb[2 * DT][32];
+  const int b = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int node = blockIdx.x, l = node * 32 + warp;
+  const int p = l * KNNT_LEAF + lane;
+  const bool on = l < nleaf && p < M;
+  const int j = on ? __ldg(vals + (long)b * M + p) : 0;
+  float* lb = lbox + ((long)b * gridDim.x + node) * (2 * DT * 32);
+#pragma unroll
+  for (int i = 0; i < DT; ++i) {
+    const float v = on ? __ldg(ref + ((long)b * DT + i) * M + j) : INFINITY;
+    float lo = on ? v : INFINITY, hi = on ? v : -INFINITY;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {  // (fminf / fmaxf leave NaN coordinates out)
+      lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+      hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+    }
+    if (lane == 0) {
+      lb[i * 32 + warp] = sb[i][warp] = lo;
+      lb[(DT + i) * 32 + warp] = sb[DT + i][warp] = hi;
+    }
+    if (l < nleaf) leaves[((long)b * nleaf + l) * ((DT + 1) * KNNT_LEAF) + i * KNNT_LEAF + lane] = v;
+  }
+  if (l < nleaf)
+    reinterpret_cast<int*>(leaves)[((long)b * nleaf + l) * ((DT + 1) * KNNT_LEAF) + DT * KNNT_LEAF + lane] = j;
+  if (lane == 0 && l + 64 < nleaf && __ldg(keys + (long)b * M + p) == __ldg(keys + (long)b * M + p + 64 * KNNT_LEAF))
+    atomicAdd(crowded, 1);
+  __syncthreads();
+  if (warp == 0) {
+    float* nb = nbox + ((long)b * ngroup + (node >> 5)) * (2 * DT * 32) + (node & 31);
+#pragma unroll
+    for (int i = 0; i < DT; ++i) {
+      float lo = sb[i][lane], hi = sb[DT + i][lane];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+        hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+      }
+      if (lane == 0) { nb[i * 32] = lo; nb[(DT + i) * 32] = hi; }
+    }
+  }
+}
+
+// Boxes of the groups, one warp per 32 nodes; also empties the slots behind the last node and group.
+template <int DT>
+__global__ void __launch_bounds__(32) knn_groups_kernel(float* __restrict__ nbox, int nnode, int ngroup,
+                                                        float* __restrict__ gbox) {
+  const int b = blockIdx.y, lane = threadIdx.x, g = blockIdx.x;
+  float* nb = nbox + ((long)b * ngroup + g) * (2 * DT * 32) + lane;  // (not read for g >= ngroup)
+  float* gb = gbox + ((long)b * (gridDim.x / 32) + (g >> 5)) * (2 * DT * 32) + (g & 31);
+  const bool on = g * 32 + lane < nnode;
+#pragma unroll
+  for (int i = 0; i < DT; ++i) {
+    float lo = on ? nb[i * 32] : INFINITY, hi = on ? nb[(DT + i) * 32] : -INFINITY;
+    if (!on && g < ngroup) { nb[i * 32] = INFINITY; nb[(DT + i) * 32] = -INFINITY; }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+      hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+    }
+    if (lane == 0) { gb[i * 32] = lo; gb[(DT + i) * 32] = hi; }
+  }
+}
+
+// Squared gap between a point and this lane's box of 32 siblings, formed like a point distance.
+template <int DT>
+__device__ __forceinline__ float box_gap2(const float (&q)[DT], const float* __restrict__ bx) {
+  float s = 0.f;
+#pragma unroll
+  for (int i = 0; i < DT; ++i) {
+    const float t = fmaxf(fmaxf(__ldg(bx + i * 32) - q[i], q[i] - __ldg(bx + (DT + i) * 32)), 0.f);
+    s = fmaf(t, t, s);
+  }
+  return s;
+}
+
+// Lane with the smallest gap if that is within thr, else -1; its gap is struck out.
+__device__ __forceinline__ int pop_nearest(float& gap, float thr, int lane) {
+  const unsigned m = __reduce_min_sync(0xffffffffu, __float_as_uint(gap));  // (gaps are >= 0)
+  if (m >= 0x7f800000u || __uint_as_float(m) > thr) return -1;
+  const int src = __ffs(__ballot_sync(0xffffffffu, __float_as_uint(gap) == m)) - 1;
+  if (lane == src) gap = INFINITY;
+  return src;
+}
+
+// qkeys: sorted keys of the queries; null: the queries are the references themselves, and a query's place
+// in the order is its leaf slot.
+template <int DT>
+__global__ void __launch_bounds__(KNNT_WARPS * 32) knn_tree_kernel(
+    const float* __restrict__ query, int M, int N, int k, int nleaf, int nnode, int ngroup,
+    const unsigned* __restrict__ keys, const unsigned* __restrict__ qkeys, const int* __restrict__ qvals,
+    const float* __restrict__ leaves, const float* __restrict__ lbox, const float* __restrict__ nbox,
+    const float* __restrict__ gbox, KnnGate gate, int64_t* __restrict__ idx, float* __restrict__ dist) {
+  if (!gate.tree()) return;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int b = blockIdx.y;
+  constexpr int LSTRIDE = (DT + 1) * KNNT_LEAF, BSTRIDE = 2 * DT * 32;
+  const float* lf = leaves + (long)b * nleaf * LSTRIDE + lane;
+  const float* lb = lbox + (long)b * nnode * BSTRIDE + lane;
+  const float* nb = nbox + (long)b * ngroup * BSTRIDE + lane;
+  const float* gb = gbox + (long)b * ((ngroup + 31) / 32) * BSTRIDE + lane;
+  const int pos = blockIdx.x * KNNT_WARPS + warp;
+  if (pos >= N) return;
+  const int n = __ldg(qvals + (long)b * N + pos);
+  float q[DT];
+#pragma unroll
+  for (int i = 0; i < DT; ++i) q[i] = __ldg(query + ((long)b * DT + i) * N + n);
+  // where the query stands among the references: that leaf comes first
+  int at = pos / KNNT_LEAF;
+  if (qkeys) {
+    const unsigned key = (__ldg(qkeys + (long)b * N + pos) & ((1u << KNNT_BITS) - 1)) | (unsigned)b << KNNT_BITS;
+    const unsigned* ks = keys + (long)b * M;
+    int lo = 0, len = M;  // lower bound, 32 probes at a time
+    while (len > 0) {
+      const int step = (len + 31) / 32;
+      const int p = lane * step;
+      const bool below = p < len && __ldg(ks + lo + p) < key;
+      const int c = __popc(__ballot_sync(0xffffffffu, below));
+      if (c == 0) break;
+      lo += (c - 1) * step + 1;
+      len = min(step - 1, len - (c - 1) * step - 1);
+    }
+    at = min(lo, M - 1) / KNNT_LEAF;
+  }
+  auto point = [&](int l, float& s, int& j) {  // this lane's reference of leaf l
+    const float* p = lf + (long)l * LSTRIDE;
+    s = 0.f;
+#pragma unroll
+    for (int i = 0; i < DT; ++i) {
+      const float t = __ldg(p + i * KNNT_LEAF) - q[i];
+      s = fmaf(t, t, s);
+    }
+    j = __float_as_int(__ldg(p + DT * KNNT_LEAF));
+  };
+  WarpTopK top;
+  float s;
+  int j;
+  point(at, s, j);
+  top.fill(s, j, k, lane);
+  // Nearest box first on every level: a leaf may hold points from both sides of a jump of the curve, so
+  // that the first k-th distance is far too large for a few queries, and these would visit thousands
+  // of leaves in index order (4 x the time of the whole search).
+  // (a NaN coordinate is at no distance from anything: the list stays empty, and no box may be asked -
+  // NaN would pass for a gap of zero, in empty slots as well)
+  bool nan = false;
+#pragma unroll
+  for (int i = 0; i < DT; ++i) nan |= q[i] != q[i];
+  for (int g0 = 0; g0 < ngroup && !nan; g0 += 32) {
+    float ggap = box_gap2<DT>(q, gb + (g0 / 32) * BSTRIDE);
+    for (int gs; (gs = pop_nearest(ggap, top.thr, lane)) >= 0;) {
+      const int n0 = (g0 + gs) * 32;
+      float ngap = box_gap2<DT>(q, nb + (long)(g0 + gs) * BSTRIDE);
+      for (int ns; (ns = pop_nearest(ngap, top.thr, lane)) >= 0;) {
+        const int l0 = (n0 + ns) * 32;
+        float lgap = box_gap2<DT>(q, lb + (long)(n0 + ns) * BSTRIDE);
+        if (l0 + lane == at) lgap = INFINITY;
+        for (int ls; (ls = pop_nearest(lgap, top.thr, lane)) >= 0;) {
+          point(l0 + ls, s, j);
+          top.offer<false>(s, j, k, lane);
+        }
+      }
+    }
+  }
+  if (lane < k) knn_store(idx, dist, ((long)b * k + lane) * N + n, top.d, top.i);
+}
+
+struct KnnTreeWs {
+  size_t bounds, keys_in, keys, vals_in, vals, leaves, lbox, nbox, gbox, cub, cub_bytes, total;
+  long items;
+  int nleaf, nnode, ngroup, end_bit;
+};
+
+static KnnTreeWs knn_tree_layout(int B, int D, int M, int N, bool same) {
+  KnnTreeWs L;
+  L.items = (long)B * M + (same ? 0 : (long)B * N);
+  L.nleaf = (M + KNNT_LEAF - 1) / KNNT_LEAF;
+  L.nnode = (L.nleaf + 31) / 32;
+  L.ngroup = (L.nnode + 31) / 32;
+  L.end_bit = KNNT_BITS;
+  while ((1L << (L.end_bit - KNNT_BITS)) < (same ? B : 2L * B)) ++L.end_bit;
+  size_t o = 0;
+  auto take = [&](size_t n) { const size_t at = o; o += (n + 255) & ~(size_t)255; return at; };
+  L.bounds = take((size_t)B * 2 * D * 4 + 16);  // (and the count of crowded leaves)
+  L.keys_in = take((size_t)L.items * 4);
+  L.keys = take((size_t)L.items * 4);
+  L.vals_in = take((size_t)L.items * 4);
+  L.vals = take((size_t)L.items * 4);
+  L.leaves = take((size_t)B * L.nleaf * (D + 1) * KNNT_LEAF * 4);
+  L.lbox = take((size_t)B * L.nnode * 2 * D * 128);
+  L.nbox = take((size_t)B * L.ngroup * 2 * D * 128);
+  L.gbox = take((size_t)B * ((L.ngroup + 31) / 32) * 2 * D * 128);
+  L.cub_bytes = 0;
+  cub::DeviceRadixSort::SortPairs(nullptr, L.cub_bytes, (const unsigned*)nullptr, (unsigned*)nullptr,
+                                  (const int*)nullptr, (int*)nullptr, (int)L.items, 0, L.end_bit);
+  L.cub = take(L.cub_bytes);
+  L.total = o;
+  return L;
+}
+
+template <int DT>
+static void knn_brute_launch(const float* ref, const float* query, int B, int D, int M, int N, int k,
+                             int64_t* idx, float* dist, cudaStream_t st, KnnGate gate = {nullptr, 0});
+
+template <int DT>
+static int knn_tree_launch(const float* ref, const float* query, int B, int M, int N, int k, int64_t* idx,
+                           float* dist, void* ws, size_t ws_bytes, cudaStream_t st) {
+  const bool same = ref == query && M == N;
+  const KnnTreeWs L = knn_tree_layout(B, DT, M, N, same);
+  if (!ws || ws_bytes < L.total) return MC_ERR_WORKSPACE;
+  if (((uintptr_t)ws) & 15) return MC_ERR_BAD_ARG;
+  uint8_t* p = (uint8_t*)ws;
+  unsigned *bounds = (unsigned*)(p + L.bounds), *keys_in = (unsigned*)(p + L.keys_in), *keys = (unsigned*)(p + L.keys);
+  int *vals_in = (int*)(p + L.vals_in), *vals = (int*)(p + L.vals);
+  float *leaves = (float*)(p + L.leaves), *lbox = (float*)(p + L.lbox), *nbox = (float*)(p + L.nbox),
+        *gbox = (float*)(p + L.gbox);
+  int* crowded = (int*)(bounds + (long)B * 2 * DT);
+  if (cudaMemsetAsync(bounds, 0, (size_t)B * 2 * DT * 4 + 4, st) != cudaSuccess) return MC_ERR_LAUNCH;
+  int bb = (M + 1023) / 1024;
+  if (bb > 148) bb = 148;
+  knn_bounds_kernel<DT><<<dim3(bb, B), 256, 0, st>>>(ref, M, bounds), MC_COUNT(1);
+  knn_keys_kernel<DT><<<grid_for(L.items, 256), 256, 0, st>>>(ref, query, B, M, same ? 0 : N, bounds, keys_in, vals_in),
+      MC_COUNT(1);
+  size_t cb = L.cub_bytes;
+  if (cub::DeviceRadixSort::SortPairs(p + L.cub, cb, keys_in, keys, vals_in, vals, (int)L.items, 0, L.end_bit, st) !=
+      cudaSuccess)
+    return MC_ERR_LAUNCH;
+  knn_leaves_kernel<DT><<<dim3(L.nnode, B), 1024, 0, st>>>(ref, M, L.nleaf, keys, vals, leaves, lbox, nbox, L.ngroup,
+                                                           crowded), MC_COUNT(1);
+  knn_groups_kernel<DT><<<dim3((L.ngroup + 31) / 32 * 32, B), 32, 0, st>>>(nbox, L.nnode, L.ngroup, gbox), MC_COUNT(1);
+  const KnnGate gate = {crowded, L.nleaf * B};
+  const unsigned* qkeys = same ? nullptr : keys + (long)B * M;
+  const int* qvals = same ? vals : vals + (long)B * M;
+  // one query per warp: queries cost between one and several times the average, and a warp (or a block) that
+  // takes several of them makes the last wave longer (8 per warp: 298 us instead of 232 us at 163 842 x 163 842)
+  const dim3 grid((unsigned)((N + KNNT_WARPS - 1) / KNNT_WARPS), (unsigned)B);
+  knn_tree_kernel<DT><<<grid, KNNT_WARPS * 32, 0, st>>>(query, M, N, k, L.nleaf, L.nnode, L.ngroup, keys,
+                                                        qkeys, qvals, leaves, lbox, nbox, gbox, gate, idx, dist), MC_COUNT(1);
+  knn_brute_launch<DT>(ref, query, B, DT, M, N, k, idx, dist, st, gate);
+  MC_CHECK_LAUNCH();
+  return MC_OK;
+}
+
+// All pairs.  A thread per query needs about 40 us + 0.02 us per reference however few queries there are;
+// a warp per query needs about 1.5 ps per pair + 1 ns per query (a reference is loaded again for every
+// query), which is less up to some 20 000 queries.
+constexpr long KNN_WIDE_QUERIES = 20000;
+
+template <int DT>
+static void knn_brute_launch(const float* ref, const float* query, int B, int D, int M, int N, int k,
+                             int64_t* idx, float* dist, cudaStream_t st, KnnGate gate) {
+  const long queries = (long)B * N;
+  if (queries <= KNN_WIDE_QUERIES) {
+    int wpq = 1;  // enough warps for the chip, at least 16 references per lane
+    while (wpq < KNNW_MAX_WARPS && queries * wpq < 148 * 16 && M >= 2 * wpq * 32 * 16) wpq *= 2;
+    const int warps = wpq > KNNW_WARPS ? wpq : KNNW_WARPS, qpb = warps / wpq;
+    knn_wide_kernel<DT><<<dim3((unsigned)((N + qpb - 1) / qpb), (unsigned)B), warps * 32, 0, st>>>(
+        ref, query, D, M, N, k, wpq, idx, dist, gate), MC_COUNT(1);
+    return;
+  }
+  if (DT > 0 && k <= 16) {
+    constexpr int DS = DT > 0 ? DT : 1;
+    dim3 grid((unsigned)((N + KNN2_THREADS - 1) / KNN2_THREADS), (unsigned)B);
+    if (k <= 8) knn_small_d_kernel<DS, 8><<<grid, KNN2_THREADS, 0, st>>>(ref, query, M, N, k, idx, dist, gate), MC_COUNT(1);
+    else if (k <= 12) knn_small_d_kernel<DS, 12><<<grid, KNN2_THREADS, 0, st>>>(ref, query, M, N, k, idx, dist, gate), MC_COUNT(1);
+    else knn_small_d_kernel<DS, 16><<<grid, KNN2_THREADS, 0, st>>>(ref, query, M, N, k, idx, dist, gate), MC_COUNT(1);
+    return;
+  }
   dim3 grid((unsigned)((N + KNN_THREADS - 1) / KNN_THREADS), (unsigned)B);
-  if (k <= 8) knn_kernel<DT, 8><<<grid, KNN_THREADS, 0, st>>>(ref, query, D, M, N, k, idx, dist), MC_COUNT(1);
-  else if (k <= 16) knn_kernel<DT, 16><<<grid, KNN_THREADS, 0, st>>>(ref, query, D, M, N, k, idx, dist), MC_COUNT(1);
-  else knn_kernel<DT, 32><<<grid, KNN_THREADS, 0, st>>>(ref, query, D, M, N, k, idx, dist), MC_COUNT(1);
+  if (k <= 8) knn_kernel<DT, 8><<<grid, KNN_THREADS, 0, st>>>(ref, query, D, M, N, k, idx, dist, gate), MC_COUNT(1);
+  else if (k <= 16) knn_kernel<DT, 16><<<grid, KNN_THREADS, 0, st>>>(ref, query, D, M, N, k, idx, dist, gate), MC_COUNT(1);
+  else knn_kernel<DT, 32><<<grid, KNN_THREADS, 0, st>>>(ref, query, D, M, N, k, idx, dist, gate), MC_COUNT(1);
 }
 
-template <int DT>
-static void knn_launch_big_k(const float* ref, const float* query, int B, int M, int N, int k,
-                             int64_t* idx, float* dist, cudaStream_t st) {
-  knn_launch_k<DT>(ref, query, B, DT, M, N, k, idx, dist, st);
-}
-
-}  // namespace mc
-
-extern "C" int mc_knn(const float* ref, const float* query, int32_t B, int32_t D, int32_t M,
-                      int32_t N, int32_t k, int64_t* idx, float* dist, void* stream) {
-  using namespace mc;
+static int knn_check(const void* ref, const void* query, int B, int D, int M, int N, int k, const void* idx,
+                     const void* dist) {
   if (!ref || !query || !idx || !dist) return MC_ERR_BAD_ARG;
   if (B <= 0 || D <= 0 || M <= 0 || N <= 0 || k <= 0) return MC_ERR_BAD_ARG;
   if (k > 32 || D > KNN_DMAX || B > 65535) return MC_ERR_TOO_LARGE;
   if (k > M) return MC_ERR_BAD_ARG;
+  return MC_OK;
+}
+
+static bool knn_tree_shape(int B, int D, int M, int N) {
+  return D <= 3 && B <= 128 && (long)B * ((long)M + N) < (1L << 30);
+}
+
+}  // namespace mc
+
+using namespace mc;
+
+extern "C" int mc_knn(const float* ref, const float* query, int32_t B, int32_t D, int32_t M,
+                      int32_t N, int32_t k, int64_t* idx, float* dist, void* stream) {
+  const int rc = knn_check(ref, query, B, D, M, N, k, idx, dist);
+  if (rc) return rc;
   cudaStream_t st = (cudaStream_t)stream;
   switch (D) {
-    case 1: knn_small_d_launch<1>(ref, query, B, M, N, k, idx, dist, st); break;
-    case 2: knn_small_d_launch<2>(ref, query, B, M, N, k, idx, dist, st); break;
-    case 3: knn_small_d_launch<3>(ref, query, B, M, N, k, idx, dist, st); break;
-    case 4: knn_small_d_launch<4>(ref, query, B, M, N, k, idx, dist, st); break;
-    default: knn_launch_k<0>(ref, query, B, D, M, N, k, idx, dist, st); break;
+    case 1: knn_brute_launch<1>(ref, query, B, D, M, N, k, idx, dist, st); break;
+    case 2: knn_brute_launch<2>(ref, query, B, D, M, N, k, idx, dist, st); break;
+    case 3: knn_brute_launch<3>(ref, query, B, D, M, N, k, idx, dist, st); break;
+    case 4: knn_brute_launch<4>(ref, query, B, D, M, N, k, idx, dist, st); break;
+    default: knn_brute_launch<0>(ref, query, B, D, M, N, k, idx, dist, st); break;
   }
   MC_CHECK_LAUNCH();
   return MC_OK;
+}
+
+// Sorting and building the leaves take about 60 us in a dozen launches, so the search pays from some number
+// of pairs on (measured: 30 000 x 2 000 points 121 us against 133 us of all pairs, 10 000 x 3 000 109 us
+// against 88 us, 163 842 x 163 842 0.31 ms against 7.65 ms).
+constexpr double KNN_TREE_PAIRS = 5e7;
+
+extern "C" size_t mc_knn_workspace_bytes(int32_t B, int32_t D, int32_t M, int32_t N, int32_t k) {
+  if (B <= 0 || D <= 0 || M <= 0 || N <= 0 || k <= 0 || k > 32 || !knn_tree_shape(B, D, M, N)) return 0;
+  if ((double)B * M * N < KNN_TREE_PAIRS || M < 32 * KNNT_LEAF) return 0;
+  return knn_tree_layout(B, D, M, N, false).total;
+}
+
+extern "C" int mc_knn_ws(const float* ref, const float* query, int32_t B, int32_t D, int32_t M, int32_t N,
+                         int32_t k, int64_t* idx, float* dist, void* ws, size_t ws_bytes, void* stream) {
+  if (!ws) return mc_knn(ref, query, B, D, M, N, k, idx, dist, stream);
+  const int rc = knn_check(ref, query, B, D, M, N, k, idx, dist);
+  if (rc) return rc;
+  if (!knn_tree_shape(B, D, M, N)) return MC_ERR_UNSUPPORTED;
+  cudaStream_t st = (cudaStream_t)stream;
+  switch (D) {
+    case 1: return knn_tree_launch<1>(ref, query, B, M, N, k, idx, dist, ws, ws_bytes, st);
+    case 2: return knn_tree_launch<2>(ref, query, B, M, N, k, idx, dist, ws, ws_bytes, st);
+    default: return knn_tree_launch<3>(ref, query, B, M, N, k, idx, dist, ws, ws_bytes, st);
+  }
 }

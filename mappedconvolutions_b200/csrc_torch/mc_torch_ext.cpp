@@ -773,8 +773,10 @@ std::vector<Tensor> knn_forward(const Tensor& ref, const Tensor& query, int64_t 
   Tensor idx = at::empty({B, k, N}, ref.options().dtype(at::kLong));
   Tensor dist = at::empty({B, k, N}, ref.options());
   c10::cuda::CUDAGuard guard(dev);
-  check(mc_knn(ref.data_ptr<float>(), query.data_ptr<float>(), (int32_t)B, (int32_t)D, (int32_t)M,
-               (int32_t)N, (int32_t)k, idx.data_ptr<int64_t>(), dist.data_ptr<float>(), cur_stream()));
+  Scratch ws = scratch(mc_knn_workspace_bytes((int32_t)B, (int32_t)D, (int32_t)M, (int32_t)N, (int32_t)k), dev);
+  check(mc_knn_ws(ref.data_ptr<float>(), query.data_ptr<float>(), (int32_t)B, (int32_t)D, (int32_t)M,
+                  (int32_t)N, (int32_t)k, idx.data_ptr<int64_t>(), dist.data_ptr<float>(), ws.p, ws.n,
+                  cur_stream()));
   return {idx, dist};
 }
 

@@ -709,8 +709,9 @@ def knn_forward(ref, query, k):
     idx = torch.empty((B, k, N), dtype=torch.int64, device=dev)
     dist = torch.empty((B, k, N), dtype=torch.float32, device=dev)
     with torch.cuda.device(dev):
-        check(lib().mc_knn(ref.data_ptr(), query.data_ptr(), B, D, M, N, int(k), idx.data_ptr(),
-                           dist.data_ptr(), _stream()))
+        wst, wsn, wsp = _ws(lib().mc_knn_workspace_bytes(B, D, M, N, int(k)), dev)
+        check(lib().mc_knn_ws(ref.data_ptr(), query.data_ptr(), B, D, M, N, int(k), idx.data_ptr(),
+                              dist.data_ptr(), wsp, wsn, _stream()))
     return [idx, dist]
 
 
