@@ -316,6 +316,12 @@ int mc_resample_gather(const mc_desc* d, const void* x, const void* map, const v
 int mc_resample_scatter(const mc_desc* d, const void* x, const void* map, const void* iw, void* y,
                         void* ws, size_t ws_bytes, void* stream);
 
+/* Per batch element a [rows][cols] matrix becomes [cols][dst_cols >= rows], zeros in the extra columns:
+ * NCHW -> channels-last with rows = channels, cols = pixels, and back with the roles swapped.
+ * elem_bytes: 2 or 4. */
+int mc_transpose(int32_t elem_bytes, int64_t B, int64_t rows, int64_t cols, const void* src, void* dst,
+                 int64_t dst_cols, void* stream);
+
 /* ---- k nearest neighbours -----------------------------------------------------------------
  * ref (B, D, M), query (B, D, N) float, contiguous.  idx (B, k, N) int64 holds 1-BASED reference
  * indices, ordered by (distance, index); dist (B, k, N) the Euclidean distances.

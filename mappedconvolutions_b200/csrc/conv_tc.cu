@@ -146,7 +146,8 @@ struct GemmArgs {
   float* gb;          // wgrad: (NOUT) fp32 or null
   int nsl;            // 64-wide slices of the gathered operand = K * C / 64
   int nst;            // pipeline stages
-  int ncol;           // channels of y / gy rows (a CTA works on a chunk of NOUT of them)
+  int ncol;           // output columns, a multiple of 64 (a CTA works on a chunk of NOUT of them)
+  int ocol;           // channels of y / gy rows: columns [ocol, ncol) are padding
   int full_cnt;       // producer warps that arrive on a stage's "full" barrier
   int mtpg;           // wgrad: M = 128 gradient tiles per CTA (blockIdx.y picks the group)
   int relu;           // fwd: y = max(0, .) after the bias
@@ -515,7 +516,7 @@ __device__ __forceinline__ void producer_loop_map(const Source& s, const Tiling&
   }
 }
 
-// Producer warp for channel counts that are not a multiple of 64 (map mode).  The gathered axis is
+// Producer warp for channel counts that are not a multiple of 64 (inverse-map mode: a multiple of 8).  The gathered axis is
 // e = tap * C + c, cut into 64-element slices and zero-padded at the end; a lane owns 8 consecutive
 // elements of a row.  With C % 8 == 0 those lie in one tap and are fetched as 16-byte vectors like
 // in the regular producer, only with a tap of the lane's own; otherwise (e.g. the 3 input channels
@@ -543,7 +544,7 @@ __device__ __forceinline__ uint4 gather_elements8(const TapEnt* trow, const bf16
   return pack8(v);
 }
 
-template <bool PAD>
+template <bool CSR, bool PAD>
 __device__ __forceinline__ void producer_loop_packed(const Source& s, const Tiling& t, int nsl,
                                                      int nslots, int nst, uint32_t stage0,
                                                      uint32_t full0, uint32_t empty0, TapEnt* table,
@@ -577,21 +578,26 @@ __device__ __forceinline__ void producer_loop_packed(const Source& s, const Tili
       if (g0 < t.mtot) s0 = s.src + (g0 / t.npix) * s.spix * C; else t0 = zero_ent;
       if (g1 < t.mtot) s1 = s.src + (g1 / t.npix) * s.spix * C; else t1 = zero_ent;
     }
+    const int p0 = CSR ? tile_row_pixel(t, tile, r0) : 0, p1 = CSR ? tile_row_pixel(t, tile, r1) : 0;
     int e0 = sl0 * 64 + lg * 8;
     for (int sl = 0; sl < nslots; ++sl, e0 += 64) {
       const bool live = (!PAD || sl < nsl) && e0 < KC;
       uint4 ra = zero, rb = zero;
+      bool more_a = false, more_b = false;
+      int tap_k = 0, tap_c = 0;
       if (live) {
         if (vec) {
           const int k = e0 / C, c = e0 - k * C;
           RowLoad A, B;
-          issue_row<false>(t0 + k, s0 + c, C, A);
-          issue_row<false>(t1 + k, s1 + c, C, B);
+          issue_row<CSR>(t0 + k, s0 + c, C, A);
+          issue_row<CSR>(t1 + k, s1 + c, C, B);
           float2 acc[4];
           blend_row(A, acc);
           ra = pack_row(acc);
           blend_row(B, acc);
           rb = pack_row(acc);
+          more_a = CSR && A.more; more_b = CSR && B.more;
+          tap_k = k; tap_c = c;
         } else {
           ra = gather_elements8(t0, s0, C, KC, e0);
           rb = gather_elements8(t1, s1, C, KC, e0);
@@ -604,6 +610,10 @@ __device__ __forceinline__ void producer_loop_packed(const Source& s, const Tili
       const uint32_t sbase = stage0 + st * STAGE_BYTES;
       sts16(sbase + so0, ra);
       sts16(sbase + so1, rb);
+      if (CSR) {
+        if (more_a) add_list_tail(s.inv_off, s.inv_ent, C, (long)p0 * s.K + tap_k, s0 + tap_c, sbase + so0, 4);
+        if (more_b) add_list_tail(s.inv_off, s.inv_ent, C, (long)p1 * s.K + tap_k, s1 + tap_c, sbase + so1, 4);
+      }
       fence_proxy_async_smem();
       __syncwarp();
       if (lane == 0) mbar_arrive(full0 + 8u * st);
@@ -1091,7 +1101,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) conv_gemm_tc_kernel(const GemmA
     }
   }
   for (int i = threadIdx.x; i < NOUT; i += TC_THREADS)
-    bias_s[i] = a.bias ? __bfloat162float(a.bias[co0 + i]) : 0.f;
+    bias_s[i] = a.bias && co0 + i < a.ocol ? __bfloat162float(a.bias[co0 + i]) : 0.f;
   fence_proxy_async_smem();
   {  // the K zero-weight entries behind the two table halves
     uint4* z = reinterpret_cast<uint4*>((TapEnt*)(sm.extra + wbytes) + (size_t)2 * TILE_M * a.s.K);
@@ -1149,6 +1159,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) conv_gemm_tc_kernel(const GemmA
       const int row = 8 * i + (lane >> 2);
       rd_addr[i] = stg + row * 64 + (((lane & 3) ^ ((row >> 1) & 3)) << 4);
     }
+    const int left = a.ocol - co0 - (lane & 3) * 8;  // columns from this lane's first piece on that exist
     uint32_t it = 0;
     for (int tile = blockIdx.x; tile < a.t.tiles; tile += gridDim.x, ++it) {
       const uint32_t acc = it & 1, aph = (it >> 1) & 1;
@@ -1160,7 +1171,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) conv_gemm_tc_kernel(const GemmA
         int img;
         bool valid;
         tile_pixel(a.t, tile, q * 32 + 8 * i + (lane >> 2), gp, img, p, valid);
-        orow[i] = valid ? a.y + gp * a.ncol + co0 + (lane & 3) * 8 : nullptr;
+        orow[i] = valid ? a.y + gp * a.ocol + co0 + (lane & 3) * 8 : nullptr;
       }
       {
         int okt = 1;
@@ -1204,7 +1215,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) conv_gemm_tc_kernel(const GemmA
           asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
                        : "=r"(o.x), "=r"(o.y), "=r"(o.z), "=r"(o.w)
                        : "r"(rd_addr[i]));
-          if (orow[i]) *reinterpret_cast<uint4*>(orow[i] + cc * 32) = o;
+          if (orow[i] && cc * 32 < left) *reinterpret_cast<uint4*>(orow[i] + cc * 32) = o;
         }
         __syncwarp();  // the block is read out before the next one is written
       }
@@ -1237,8 +1248,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) conv_gemm_tc_kernel(const GemmA
       producer_rowwise<false>(a.s, a.t, a.nsl, a.nsl, nst, stage0, full_bar(0), empty_bar(0),
                               (TapEnt*)(sm.extra + wbytes), abort_flag, warp - FIRST_PROD_WARP, lane,
                               0x36);
-    } else if (!CSR && a.s.packed) {
-      producer_loop_packed<false>(a.s, a.t, a.nsl, a.nsl, nst, stage0, full_bar(0), empty_bar(0),
+    } else if (a.s.packed) {
+      producer_loop_packed<CSR, false>(a.s, a.t, a.nsl, a.nsl, nst, stage0, full_bar(0), empty_bar(0),
                                   (TapEnt*)(sm.extra + wbytes), tabbar0, abort_flag,
                                   warp - FIRST_PROD_WARP, lane, 0x35);
     } else if (a.s.interp == 0) {
@@ -1392,8 +1403,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) conv_wgrad_tc_kernel(const Gemm
             int img;
             bool valid;
             tile_pixel(a.t, tile, r, gp, img, p, valid);
-            v[i] = valid ? ldcg16(a.gy + gp * a.ncol + co0 + nb * 64 + lg * 8)
-                         : make_uint4(0, 0, 0, 0);
+            v[i] = valid && co0 + nb * 64 + lg * 8 < a.ocol ? ldcg16(a.gy + gp * a.ocol + co0 + nb * 64 + lg * 8)
+                                                            : make_uint4(0, 0, 0, 0);
           }
 #pragma unroll
           for (int i = 0; i < TILE_M / (N_EPI_WARPS * 4); ++i) {
@@ -1416,8 +1427,9 @@ __global__ void __launch_bounds__(TC_THREADS, 1) conv_wgrad_tc_kernel(const Gemm
           tile_pixel(a.t, tile, r, gp, img, p, valid);
 #pragma unroll
           for (int nb = 0; nb < NOUT / 64; ++nb) {
-            const uint4 v = valid ? ldcg16(a.gy + gp * a.ncol + co0 + nb * 64 + lg * 8)
-                                  : make_uint4(0, 0, 0, 0);
+            const uint4 v = valid && co0 + nb * 64 + lg * 8 < a.ocol
+                                ? ldcg16(a.gy + gp * a.ocol + co0 + nb * 64 + lg * 8)
+                                : make_uint4(0, 0, 0, 0);
             // N > 64: consecutive 64-channel blocks are separate swizzle atoms, STAGE_BYTES apart
             sts16(sbase + nb * STAGE_BYTES + r * 128 + ((lg ^ (r & 7)) << 4), v);
             float* b8 = bsum + nb * 8;
@@ -1442,7 +1454,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) conv_wgrad_tc_kernel(const Gemm
     }
     asm volatile("bar.sync 1, %0;" ::"n"(N_EPI_WARPS * 32) : "memory");
     if (do_gb)
-      for (int i = lw * 32 + lane; i < NOUT; i += N_EPI_WARPS * 32) atomicAdd(a.gb + co0 + i, gb_s[i]);
+      for (int i = lw * 32 + lane; i < NOUT && co0 + i < a.ocol; i += N_EPI_WARPS * 32) atomicAdd(a.gb + co0 + i, gb_s[i]);
     // epilogue: partial weight gradient of this CTA
     if (ok && mbar_wait(done_bar, 0, abort_flag, 0x52, 1024)) {
       tc_fence_after_sync();
@@ -1461,7 +1473,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) conv_wgrad_tc_kernel(const Gemm
 #pragma unroll
             for (int c = 0; c < 32; ++c) {
               const int co = co0 + cc * 32 + c;
-              atomicAdd(a.gw + ((long)co * a.s.C + ci) * a.s.K + tap, __uint_as_float(v[c]));
+              if (co < a.ocol) atomicAdd(a.gw + ((long)co * a.s.C + ci) * a.s.K + tap, __uint_as_float(v[c]));
             }
           }
         }
@@ -1482,7 +1494,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) conv_wgrad_tc_kernel(const Gemm
                              (TapEnt*)(sm.extra + (size_t)GY_STAGES * GYB), abort_flag,
                              warp - FIRST_PROD_WARP, lane, 0x64);
     } else if (a.s.packed) {
-      producer_loop_packed<true>(a.s, a.t, nsl, nsl_pad, nst, stage0, full_bar(0), empty_bar(0),
+      producer_loop_packed<false, true>(a.s, a.t, nsl, nsl_pad, nst, stage0, full_bar(0), empty_bar(0),
                                  (TapEnt*)(sm.extra + (size_t)GY_STAGES * GYB), tabbar0,
                                  abort_flag, warp - FIRST_PROD_WARP, lane, 0x63, sl0);
     } else if (a.s.interp == 0) {
@@ -1517,20 +1529,21 @@ __global__ void __launch_bounds__(TC_THREADS, 1) conv_wgrad_tc_kernel(const Gemm
 // transpose = 0 (forward): rows = output channels, slices run over (tap, input-channel block).
 // transpose = 1 (dgrad)  : rows = input channels,  slices run over (tap, output-channel block).
 // The reduction axis is e = tap * red + r, cut into 64-element slices and zero-padded at the end.
+// `rows` real rows of `rows_img` (a multiple of 64); the others are zero.
 __global__ void weight_image_kernel(const bf16* __restrict__ w, uint16_t* __restrict__ img, int rows,
-                                    int red, int K, int transpose, int Cin_w) {
+                                    int rows_img, int red, int K, int transpose, int Cin_w) {
   const int nsl = (K * red + 63) / 64;
-  const long total = (long)nsl * rows * 64;
+  const long total = (long)nsl * rows_img * 64;
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < total;
        i += (long)gridDim.x * blockDim.x) {
     const int c = (int)(i % 64);
-    const int n = (int)((i / 64) % rows);
-    const int s = (int)(i / (64L * rows));
+    const int n = (int)((i / 64) % rows_img);
+    const int s = (int)(i / (64L * rows_img));
     const int e = s * 64 + c;
     const int tap = e / red, r = e - tap * red;
     const long src = transpose ? ((long)r * Cin_w + n) * K + tap : ((long)n * Cin_w + r) * K + tap;
-    const long dst = (long)s * rows * 64 + (long)n * 64 + ((((c >> 3) ^ (n & 7)) << 3) | (c & 7));
-    img[dst] = e < K * red ? reinterpret_cast<const uint16_t*>(w)[src] : (uint16_t)0;
+    const long dst = (long)s * rows_img * 64 + (long)n * 64 + ((((c >> 3) ^ (n & 7)) << 3) | (c & 7));
+    img[dst] = e < K * red && n < rows ? reinterpret_cast<const uint16_t*>(w)[src] : (uint16_t)0;
   }
 }
 
@@ -1765,11 +1778,17 @@ static bool plan_gemm(int ncol, int nsl, int K, GemmPlan& p) {
 // 64-element slices of the gathered (tap, input channel) axis of forward / wgrad
 static int fwd_slices(const mc_desc* d) { return (int)(((long)d->K * d->C_in + 63) / 64); }
 
+// Output columns of the MMA tiles: channel counts (multiples of 8) that are not a multiple of 64 are padded (zero weights,
+// columns that are not stored), which wastes at most seven eighths of the MMA work; the CUDA-core kernels they would
+// otherwise take run at a hundredth of the rate
+// (128 -> 96 channels on 3 x 433 x 866 pixels: 50.7 ms).
+static int pad64(int c) { return (c + 63) & ~63; }
+
 bool conv_tc_fwd_supported(const mc_desc* d) {
   if (d->dtype != MC_BF16 || d->layout != MC_NHWC || d->P != 0) return false;
-  if ((long)d->K * d->C_in >= (1L << 24)) return false;
+  if (d->C_out % 8 != 0 || (long)d->K * d->C_in >= (1L << 24)) return false;
   GemmPlan p;
-  return plan_gemm(d->C_out, fwd_slices(d), d->K, p);
+  return plan_gemm(pad64(d->C_out), fwd_slices(d), d->K, p);
 }
 
 // Streamed weights need the prebuilt tap table; when the caller passes the raw sample map the
@@ -1780,12 +1799,12 @@ static bool rowwise_shape(const mc_desc* d) { return d->C_in % 64 != 0 && (long)
 
 static bool fwd_needs_table(const mc_desc* d) {
   GemmPlan p;
-  if (!plan_gemm(d->C_out, fwd_slices(d), d->K, p)) return false;
+  if (!plan_gemm(pad64(d->C_out), fwd_slices(d), d->K, p)) return false;
   return !p.wres || (rowwise_shape(d) && p.nst >= ROW_TEAMS);
 }
 
 size_t conv_tc_fwd_wimg_bytes(const mc_desc* d) {
-  return ((size_t)fwd_slices(d) * 64 * d->C_out * sizeof(bf16) + 255) & ~(size_t)255;
+  return ((size_t)fwd_slices(d) * 64 * pad64(d->C_out) * sizeof(bf16) + 255) & ~(size_t)255;
 }
 
 size_t tapmap_bytes(const mc_desc* d);
@@ -1882,7 +1901,7 @@ int tapmap_build_weighted_launch(const mc_desc* d, const void* map, const void* 
 static int fwd_launch_impl(const mc_desc* d, const void* x, const void* map, const void* tab,
                            const void* w, const void* bias, void* y, void* ws, size_t ws_bytes,
                            cudaStream_t st) {
-  if (!ws || ws_bytes < (tab ? (size_t)fwd_slices(d) * 64 * d->C_out * sizeof(bf16) : conv_tc_fwd_ws(d)))
+  if (!ws || ws_bytes < (tab ? (size_t)fwd_slices(d) * 64 * pad64(d->C_out) * sizeof(bf16) : conv_tc_fwd_ws(d)))
     return MC_ERR_WORKSPACE;
   if (!aligned16(x) || !aligned16(y) || !aligned16(ws) || !aligned16(map) || !aligned16(tab))
     return MC_ERR_BAD_ARG;
@@ -1898,13 +1917,14 @@ static int fwd_launch_impl(const mc_desc* d, const void* x, const void* map, con
   a.nsl = fwd_slices(d);
   a.s.KC = d->K * d->C_in;
   a.s.packed = d->C_in % 64 != 0;
-  a.ncol = d->C_out;
+  a.ocol = d->C_out;
+  a.ncol = pad64(d->C_out);
   a.relu = (d->flags & MC_FLAG_RELU) ? 1 : 0;
   GemmPlan p;
   if (!plan_gemm(a.ncol, a.nsl, d->K, p)) return MC_ERR_UNSUPPORTED;
   a.nst = p.nst;
-  const long nw = (long)a.nsl * 64 * d->C_out;
-  weight_image_kernel<<<grid_for(nw, 256), 256, 0, st>>>((const bf16*)w, (uint16_t*)ws, d->C_out,
+  const long nw = (long)a.nsl * 64 * a.ncol;
+  weight_image_kernel<<<grid_for(nw, 256), 256, 0, st>>>((const bf16*)w, (uint16_t*)ws, d->C_out, a.ncol,
                                                          d->C_in, d->K, 0, d->C_in), MC_COUNT(1);
   if (!tab && fwd_needs_table(d)) {  // build the table behind the weight image
     void* t = (uint8_t*)ws + conv_tc_fwd_wimg_bytes(d);
@@ -2008,16 +2028,21 @@ int invmap_build_launch(const mc_desc* d_in, const void* map, const void* iw, vo
 
 // ---- dgrad through the inverse map ---------------------------------------------------------------------
 
+// 64-element slices of the gathered (tap, output channel) axis of the input gradient
+static int dgrad_slices(const mc_desc* d) { return (int)(((long)d->K * d->C_out + 63) / 64); }
+
 bool conv_tc_dgrad_supported(const mc_desc* d) {
   if (d->dtype != MC_BF16 || d->layout != MC_NHWC || d->P != 0) return false;
-  if (d->C_out % 64 != 0) return false;
+  // (channels in 16-byte pieces on both sides; an image with fewer than 8 channels would also leave nearly all
+  // of the 64 output columns empty)
+  if (d->C_out % 8 != 0 || d->C_in % 8 != 0 || (long)d->K * d->C_out >= (1L << 24)) return false;
   if (!invmap_supported(d)) return false;
   GemmPlan p;
-  return plan_gemm(d->C_in, d->K * (d->C_out / 64), d->K, p);
+  return plan_gemm(pad64(d->C_in), dgrad_slices(d), d->K, p);
 }
 
 size_t conv_tc_dgrad_ws(const mc_desc* d) {
-  return (size_t)d->K * d->C_in * d->C_out * sizeof(bf16);
+  return (size_t)dgrad_slices(d) * 64 * pad64(d->C_in) * sizeof(bf16);
 }
 
 int conv_tc_dgrad_launch(const mc_desc* d, const void* gy, const void* inv, const void* w,
@@ -2034,15 +2059,18 @@ int conv_tc_dgrad_launch(const mc_desc* d, const void* gy, const void* inv, cons
   if ((long)d->B * d->OH * d->OW >= (1L << 30)) return MC_ERR_TOO_LARGE;
   if (!make_tiling(a.t, d->B, d->IH, d->IW)) return MC_ERR_TOO_LARGE;
   a.wimg = (const uint4*)ws; a.bias = (const bf16*)bias_out; a.y = (bf16*)gx;
-  a.nsl = d->K * (d->C_out / 64);
-  a.ncol = d->C_in;
+  a.nsl = dgrad_slices(d);
+  a.s.KC = d->K * d->C_out;
+  a.s.packed = d->C_out % 64 != 0;
+  a.ocol = d->C_in;
+  a.ncol = pad64(d->C_in);
   a.relu = (bias_out && (d->flags & MC_FLAG_RELU)) ? 1 : 0;  // the transposed layer's forward
   GemmPlan p;
   if (!plan_gemm(a.ncol, a.nsl, d->K, p)) return MC_ERR_UNSUPPORTED;
   a.nst = p.nst;
   a.full_cnt = N_PRODUCER_WARPS;
-  const long nw = (long)d->K * d->C_in * d->C_out;
-  weight_image_kernel<<<grid_for(nw, 256), 256, 0, st>>>((const bf16*)w, (uint16_t*)ws, d->C_in,
+  const long nw = (long)a.nsl * 64 * a.ncol;
+  weight_image_kernel<<<grid_for(nw, 256), 256, 0, st>>>((const bf16*)w, (uint16_t*)ws, d->C_in, a.ncol,
                                                          d->C_out, d->K, 1, d->C_in), MC_COUNT(1);
   return launch_gemm<true>(a, p, true, st);
 }
@@ -2058,11 +2086,11 @@ struct WgradPlan {
 };
 
 static bool plan_wgrad(const mc_desc* d, WgradPlan& p) {
-  if (d->C_out % 64 != 0 || (long)d->K * d->C_in >= (1L << 24)) return false;
+  if (d->C_out % 8 != 0 || (long)d->K * d->C_in >= (1L << 24)) return false;
   const int nsl = fwd_slices(d);
   const int nmt = (nsl + 1) / 2;
-  p.nout = d->C_out % 128 == 0 ? 128 : 64;
-  p.chunks = d->C_out / p.nout;
+  p.nout = pad64(d->C_out) % 128 == 0 ? 128 : 64;
+  p.chunks = pad64(d->C_out) / p.nout;
   const int cap = 512 / p.nout;
   p.groups = (nmt + cap - 1) / cap;
   p.mtpg = (nmt + p.groups - 1) / p.groups;
@@ -2116,7 +2144,8 @@ static int wgrad_launch_impl(const mc_desc* d, const void* gy, const void* x, co
   a.nsl = fwd_slices(d);
   a.s.KC = d->K * d->C_in;
   a.s.packed = d->C_in % 64 != 0;
-  a.ncol = d->C_out;
+  a.ocol = d->C_out;
+  a.ncol = pad64(d->C_out);
   WgradPlan p;
   if (!plan_wgrad(d, p)) return MC_ERR_UNSUPPORTED;
   a.nst = p.nst;
@@ -2174,7 +2203,7 @@ extern "C" int mc_conv_fwd_static_scratch(const mc_desc* d, const void* x, const
   int rc = check_conv_desc_public(d);
   if (rc) return rc;
   if (!x || !map || !w || !y) return MC_ERR_BAD_ARG;
-  if (!conv_tc_fwd_supported(d)) return MC_ERR_UNSUPPORTED;
+  if (!conv_tc_fwd_supported(d) || d->C_out % 64 != 0) return MC_ERR_UNSUPPORTED;
   if (conv_tc_fwd_ws(d) > STATIC_SCRATCH_BYTES) return MC_ERR_TOO_LARGE;
   int dev = -1;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= STATIC_SCRATCH_MAX_DEVICES)

@@ -57,8 +57,10 @@ int layout_of(const Tensor& x) {
   TORCH_CHECK(false, "input must be contiguous");
 }
 
+Tensor channels_last(const Tensor& t);
+Tensor channels_first(const Tensor& t);
 Tensor as_layout(const Tensor& t, int layout) {
-  return layout == MC_NHWC ? t.contiguous(at::MemoryFormat::ChannelsLast) : t.contiguous();
+  return layout == MC_NHWC ? channels_last(t) : channels_first(t);
 }
 
 Tensor empty_in(at::IntArrayRef shape, const Tensor& like, int layout,
@@ -310,7 +312,30 @@ std::vector<int64_t> plan_cache_kinds() {
   return kinds;
 }
 
-Tensor channels_last(const Tensor& t) { return t.contiguous(at::MemoryFormat::ChannelsLast); }
+// NCHW -> channels-last and back with the library's own transpose (torch's strided copy takes four times as
+// long); anything else - other dtypes, tensors contiguous in neither layout - through torch.
+Tensor channels_last(const Tensor& t) {
+  const auto esz = t.element_size();
+  if (t.dim() != 4 || !t.is_cuda() || t.numel() == 0 || !t.is_contiguous() ||
+      t.is_contiguous(at::MemoryFormat::ChannelsLast) || (esz != 2 && esz != 4))
+    return t.contiguous(at::MemoryFormat::ChannelsLast);
+  Tensor out = at::empty(t.sizes(), t.options(), at::MemoryFormat::ChannelsLast);
+  c10::cuda::CUDAGuard guard(t.device());
+  check(mc_transpose((int32_t)esz, t.size(0), t.size(1), t.size(2) * t.size(3), t.data_ptr(), out.data_ptr(),
+                     t.size(1), cur_stream()));
+  return out;
+}
+Tensor channels_first(const Tensor& t) {
+  const auto esz = t.element_size();
+  if (t.dim() != 4 || !t.is_cuda() || t.numel() == 0 || t.is_contiguous() ||
+      !t.is_contiguous(at::MemoryFormat::ChannelsLast) || (esz != 2 && esz != 4))
+    return t.contiguous();
+  Tensor out = at::empty(t.sizes(), t.options());
+  c10::cuda::CUDAGuard guard(t.device());
+  check(mc_transpose((int32_t)esz, t.size(0), t.size(2) * t.size(3), t.size(1), t.data_ptr(), out.data_ptr(),
+                     t.size(2) * t.size(3), cur_stream()));
+  return out;
+}
 
 // The tensor-core kernels read rows with 16-byte vector loads and bulk copies.  A view into a larger
 // tensor (a batch slice, a map slice) can start on any element boundary: such a tensor is copied
@@ -351,8 +376,7 @@ Tensor conv_forward(const Tensor& input_in, const Tensor& sample_map_in, const O
   const int64_t Cout = weight.size(0), OH = sample_map.size(0), OW = sample_map.size(1);
   if (!nhwc && via_channels_last(input, iw, make_desc(input.scalar_type(), MC_NHWC, B, Cin, Cout, IH,
                                                       IW, OH, OW, K, 0, interp)))
-    return conv_forward(channels_last(input), sample_map, iw, weight, bias, K, interp, true,
-                        relu).contiguous();
+    return channels_first(conv_forward(channels_last(input), sample_map, iw, weight, bias, K, interp, true, relu));
   const int layout = nhwc ? MC_NHWC : layout_of(input);
   check_map(input, sample_map, iw);
   TORCH_CHECK(weight.is_contiguous() && bias.is_contiguous(), "weight and bias must be contiguous");
@@ -440,7 +464,7 @@ std::vector<Tensor> conv_backward(const Tensor& grad_output_in, const Tensor& sa
     auto g = conv_backward(channels_last(grad_output_in), sample_map, iw,
                            channels_last(input), weight, bias, K, interp, need_input_grad, true,
                            need_weight_grad);
-    if (g[0].defined()) g[0] = g[0].contiguous();
+    if (g[0].defined()) g[0] = channels_first(g[0]);
     return g;
   }
   const int layout = nhwc ? MC_NHWC : layout_of(input);
@@ -536,8 +560,7 @@ Tensor tconv_forward(const Tensor& input_in, const Tensor& sample_map_in, const 
   // the same layer seen as a convolution: the sampled image carries C_out channels, the grid C_in
   if (!nhwc && via_channels_last(input, iw, make_desc(input.scalar_type(), MC_NHWC, B, Cout, Cin, OHt,
                                                       OWt, H, W, K, 0, interp)))
-    return tconv_forward(channels_last(input), sample_map, iw, weight, bias, OHt, OWt, K,
-                         interp, true).contiguous();
+    return channels_first(tconv_forward(channels_last(input), sample_map, iw, weight, bias, OHt, OWt, K, interp, true));
   const int layout = nhwc ? MC_NHWC : layout_of(input);
   check_map(input, sample_map, iw);
   TORCH_CHECK(weight.is_contiguous() && bias.is_contiguous(), "weight and bias must be contiguous");
@@ -584,7 +607,7 @@ std::vector<Tensor> tconv_backward(const Tensor& grad_output_in, const Tensor& s
                                                       OWt, H, W, K, 0, interp))) {
     auto g = tconv_backward(channels_last(grad_output_in), sample_map, iw,
                             channels_last(input), weight, bias, K, interp, true);
-    g[0] = g[0].contiguous();
+    g[0] = channels_first(g[0]);
     return g;
   }
   const int layout = nhwc ? MC_NHWC : layout_of(input);
