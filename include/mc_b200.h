@@ -316,6 +316,9 @@ int mc_resample_gather(const mc_desc* d, const void* x, const void* map, const v
 int mc_resample_scatter(const mc_desc* d, const void* x, const void* map, const void* iw, void* y,
                         void* ws, size_t ws_bytes, void* stream);
 
+/* Rounds two float32 arrays (a weight and a bias gradient) to bfloat16 in one launch. */
+int mc_round_pair(const float* a, void* da, int64_t na, const float* b, void* db, int64_t nb, void* stream);
+
 /* Per batch element a [rows][cols] matrix becomes [cols][dst_cols >= rows], zeros in the extra columns:
  * NCHW -> channels-last with rows = channels, cols = pixels, and back with the roles swapped.
  * elem_bytes: 2 or 4. */

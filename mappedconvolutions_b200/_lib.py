@@ -78,6 +78,7 @@ SIGNATURES = {
     "mc_resample_gather": (ctypes.c_int, [_dp, _vp, _vp, _vp, _vp, _vp]),
     "mc_resample_scatter": (ctypes.c_int, [_dp, _vp, _vp, _vp, _vp, _vp, _sz, _vp]),
     "mc_knn": (ctypes.c_int, [_vp, _vp, _i32, _i32, _i32, _i32, _i32, _vp, _vp, _vp]),
+    "mc_round_pair": (ctypes.c_int, [_vp, _vp, ctypes.c_int64, _vp, _vp, ctypes.c_int64, _vp]),
     "mc_transpose": (ctypes.c_int, [_i32, ctypes.c_int64, ctypes.c_int64, ctypes.c_int64, _vp, _vp, ctypes.c_int64,
                                     _vp]),
     "mc_knn_workspace_bytes": (_sz, [_i32, _i32, _i32, _i32, _i32]),

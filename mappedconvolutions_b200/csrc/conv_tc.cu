@@ -2156,9 +2156,10 @@ static int wgrad_launch_impl(const mc_desc* d, const void* gy, const void* x, co
     a.full_cnt = N_PRODUCER_WARPS / ROW_TEAMS;
     a.s.tab32 = tapmap_compact(d, tab);
   }
-  if (cudaMemsetAsync(gw, 0, (size_t)d->C_out * d->C_in * d->K * sizeof(float), st) != cudaSuccess)
-    return MC_ERR_LAUNCH;
-  if (gb && cudaMemsetAsync(gb, 0, (size_t)d->C_out * sizeof(float), st) != cudaSuccess)
+  const size_t nw = (size_t)d->C_out * d->C_in * d->K;
+  const bool joined = gb == (float*)gw + nw;  // one buffer: one memset
+  if (cudaMemsetAsync(gw, 0, (nw + (joined ? d->C_out : 0)) * sizeof(float), st) != cudaSuccess) return MC_ERR_LAUNCH;
+  if (gb && !joined && cudaMemsetAsync(gb, 0, (size_t)d->C_out * sizeof(float), st) != cudaSuccess)
     return MC_ERR_LAUNCH;
   // very few input channels and a nearest map with its compact table: one pass over grad_output
   if (tab && smallcin_wgrad_shape(d) && tapmap_compact(d, tab))

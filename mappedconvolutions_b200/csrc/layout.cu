@@ -105,7 +105,25 @@ static int transpose_launch(long B, long rows, long cols, const void* src, void*
   return MC_OK;
 }
 
+// float32 sums of a weight / bias gradient -> bf16 parameters' gradients, both in one launch.
+__global__ void __launch_bounds__(256) round_pair_kernel(const float* __restrict__ a, bf16* __restrict__ da, long na,
+                                                         const float* __restrict__ b, bf16* __restrict__ db, long n) {
+  for (long i = blockIdx.x * 256L + threadIdx.x; i < n; i += gridDim.x * 256L) {
+    if (i < na) da[i] = __float2bfloat16_rn(a[i]);
+    else db[i - na] = __float2bfloat16_rn(b[i - na]);
+  }
+}
+
 }  // namespace mc
+
+extern "C" int mc_round_pair(const float* a, void* da, int64_t na, const float* b, void* db, int64_t nb, void* stream) {
+  using namespace mc;
+  if (na < 0 || nb < 0 || na + nb <= 0 || (na && (!a || !da)) || (nb && (!b || !db))) return MC_ERR_BAD_ARG;
+  round_pair_kernel<<<grid_for(na + nb, 256), 256, 0, (cudaStream_t)stream>>>(a, (bf16*)da, na, b, (bf16*)db, na + nb),
+      MC_COUNT(1);
+  MC_CHECK_LAUNCH();
+  return MC_OK;
+}
 
 extern "C" int mc_transpose(int32_t elem_bytes, int64_t B, int64_t rows, int64_t cols, const void* src, void* dst,
                             int64_t dst_cols, void* stream) {

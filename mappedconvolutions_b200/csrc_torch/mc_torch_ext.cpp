@@ -362,6 +362,30 @@ bool via_channels_last(const Tensor& input, const OptTensor& iw, mc_desc d_nhwc)
   return mc_conv_fwd_workspace_bytes(&d_nhwc) > 0;
 }
 
+// Where a weight / bias gradient is summed: float32 (float64 for double layers); for bf16 parameters both
+// sums share one buffer (one memset) and are rounded together at the end (one launch).
+struct ParamGrads {
+  Tensor gw, gb, sums;
+  void *pw = nullptr, *pb = nullptr;
+  int64_t nw = 0, nb = 0;
+  ParamGrads(const Tensor& weight, int64_t n_bias) : nw(weight.numel()), nb(n_bias) {
+    gw = at::empty(weight.sizes(), weight.options());
+    gb = at::empty({n_bias}, weight.options());
+    if (weight.scalar_type() == at::kBFloat16) {
+      sums = at::empty({nw + nb}, weight.options().dtype(at::kFloat));
+      pw = sums.data_ptr();
+      pb = sums.data_ptr<float>() + nw;
+    } else {
+      pw = gw.data_ptr();
+      pb = gb.data_ptr();
+    }
+  }
+  void finish() {
+    if (sums.defined())
+      check(mc_round_pair((const float*)pw, gw.data_ptr(), nw, (const float*)pb, gb.data_ptr(), nb, cur_stream()));
+  }
+};
+
 // ---- convolution ---------------------------------------------------------------------------------------
 
 // relu: y = max(0, conv + bias), applied in the kernel's epilogue (MC_FLAG_RELU)
@@ -477,10 +501,7 @@ std::vector<Tensor> conv_backward(const Tensor& grad_output_in, const Tensor& sa
   mc_desc f;
   const bool folded = weighted_folds(d_map, iw, &f);
   const mc_desc d = folded ? f : d_map;
-  const auto acc = input.scalar_type() == at::kDouble ? at::kDouble : at::kFloat;
   Tensor gx = need_input_grad ? empty_in(input.sizes(), input, layout) : Tensor();
-  Tensor gw = at::empty(weight.sizes(), weight.options().dtype(acc));
-  Tensor gb = at::empty({Cout}, weight.options().dtype(acc));
   c10::cuda::CUDAGuard guard(dev);
   auto rp = iw.has_value() ? std::pair<Tensor, Tensor>() : row_plan(d, sample_map);
   if (need_input_grad && rp.first.defined()) {
@@ -501,8 +522,8 @@ std::vector<Tensor> conv_backward(const Tensor& grad_output_in, const Tensor& sa
     check(mc_conv_dgrad_tapsum(&d, z.data_ptr(), inv.data_ptr(), gx.data_ptr(), cur_stream()));
     need_input_grad = false;  // done
   }
-  const size_t n_dgrad = inv.defined() ? mc_conv_dgrad_inv_workspace_bytes(&d)
-                                       : mc_conv_dgrad_workspace_bytes(&d_map);
+  const size_t n_dgrad = !need_input_grad ? 0 : inv.defined() ? mc_conv_dgrad_inv_workspace_bytes(&d)
+                                                              : mc_conv_dgrad_workspace_bytes(&d_map);
   Scratch ws = scratch(std::max(n_dgrad, mc_conv_wgrad_workspace_bytes(&d_map)), dev);
   if (!need_input_grad) {
   } else if (inv.defined()) {
@@ -513,12 +534,13 @@ std::vector<Tensor> conv_backward(const Tensor& grad_output_in, const Tensor& sa
                         weight.data_ptr(), nullptr, gx.data_ptr(), ws.p, ws.n, cur_stream()));
   }
   if (!need_weight_grad) return {gx, Tensor(), Tensor()};
+  ParamGrads pg(weight, Cout);
   if (rp.first.defined()) {  // row-invariant map: weight gradient from the same plan
     Scratch wsr = scratch(mc_conv_wgrad_rowplan_workspace_bytes(&d, rp.second.data_ptr()), dev);
     check(mc_conv_wgrad_rowplan(&d, grad_output.data_ptr(), input.data_ptr(), rp.second.data_ptr(),
-                                rp.first.data_ptr(), gw.data_ptr(), gb.data_ptr(), wsr.p, wsr.n,
-                                cur_stream()));
-    return {gx, gw.to(weight.scalar_type()), gb.to(bias.scalar_type())};
+                                rp.first.data_ptr(), pg.pw, pg.pb, wsr.p, wsr.n, cur_stream()));
+    pg.finish();
+    return {gx, pg.gw, pg.gb};
   }
   Tensor tab = folded ? tap_map_weighted(d_map, f, sample_map, *iw)
                       : (iw.has_value() ? Tensor() : tap_map(d, sample_map));
@@ -527,21 +549,22 @@ std::vector<Tensor> conv_backward(const Tensor& grad_output_in, const Tensor& sa
     const Tensor yr = aligned16(*relu_output);
     if (tab.defined())
       rc = mc_conv_wgrad_tap_relu(&d, grad_output.data_ptr(), yr.data_ptr(), input.data_ptr(), tab.data_ptr(),
-                                  gw.data_ptr(), gb.data_ptr(), cur_stream());
+                                  pg.pw, pg.pb, cur_stream());
     if (rc == MC_ERR_UNSUPPORTED)  // no kernel masks on the fly for this shape: mask first
       return conv_backward(at::threshold_backward(grad_output, yr, 0), sample_map, iw, input, weight, bias, K,
                            interp, false, nhwc, true);
     check(rc);
-    return {gx, gw.to(weight.scalar_type()), gb.to(bias.scalar_type())};
+    pg.finish();
+    return {gx, pg.gw, pg.gb};
   }
   if (tab.defined())  // weight / bias gradient on the tensor cores from the prebuilt table
-    rc = mc_conv_wgrad_tap(&d, grad_output.data_ptr(), input.data_ptr(), tab.data_ptr(),
-                           gw.data_ptr(), gb.data_ptr(), cur_stream());
+    rc = mc_conv_wgrad_tap(&d, grad_output.data_ptr(), input.data_ptr(), tab.data_ptr(), pg.pw, pg.pb, cur_stream());
   if (rc == MC_ERR_UNSUPPORTED)  // shapes only the generic kernels take
-    rc = mc_conv_wgrad(&d_map, grad_output.data_ptr(), input.data_ptr(), sample_map.data_ptr(), ptr(iw),
-                       gw.data_ptr(), gb.data_ptr(), ws.p, ws.n, cur_stream());
+    rc = mc_conv_wgrad(&d_map, grad_output.data_ptr(), input.data_ptr(), sample_map.data_ptr(), ptr(iw), pg.pw, pg.pb,
+                       ws.p, ws.n, cur_stream());
   check(rc);
-  return {gx, gw.to(weight.scalar_type()), gb.to(bias.scalar_type())};
+  pg.finish();
+  return {gx, pg.gw, pg.gb};
 }
 
 // ---- transposed convolution ------------------------------------------------------------------------------
@@ -590,7 +613,7 @@ Tensor tconv_forward(const Tensor& input_in, const Tensor& sample_map_in, const 
 std::vector<Tensor> tconv_backward(const Tensor& grad_output_in, const Tensor& sample_map_in,
                                    const OptTensor& iw, const Tensor& input_in, const Tensor& weight,
                                    const Tensor& bias, int64_t K, int64_t interp,
-                                   bool nhwc = false) {
+                                   bool nhwc = false, bool need_input_grad = true, bool need_weight_grad = true) {
   const Tensor input = aligned16(input_in), sample_map = aligned16(sample_map_in);
   TORCH_CHECK(input.dim() == 4 && weight.dim() == 3 && grad_output_in.dim() == 4,
               "input and grad_output must be 4-D, weight 3-D");
@@ -606,8 +629,8 @@ std::vector<Tensor> tconv_backward(const Tensor& grad_output_in, const Tensor& s
   if (!nhwc && via_channels_last(input, iw, make_desc(input.scalar_type(), MC_NHWC, B, Cout, Cin, OHt,
                                                       OWt, H, W, K, 0, interp))) {
     auto g = tconv_backward(channels_last(grad_output_in), sample_map, iw,
-                            channels_last(input), weight, bias, K, interp, true);
-    g[0] = channels_first(g[0]);
+                            channels_last(input), weight, bias, K, interp, true, need_input_grad, need_weight_grad);
+    if (g[0].defined()) g[0] = channels_first(g[0]);
     return g;
   }
   const int layout = nhwc ? MC_NHWC : layout_of(input);
@@ -617,10 +640,7 @@ std::vector<Tensor> tconv_backward(const Tensor& grad_output_in, const Tensor& s
                               n_interp(iw), interp);
   const mc_desc ds = make_desc(input.scalar_type(), layout, B, Cout, Cin, OHt, OWt, H, W, K,
                                n_interp(iw), interp);
-  const auto acc = input.scalar_type() == at::kDouble ? at::kDouble : at::kFloat;
-  Tensor gx = empty_in(input.sizes(), input, layout);
-  Tensor gw = at::empty(weight.sizes(), weight.options().dtype(acc));
-  Tensor gb = at::empty({Cout}, weight.options().dtype(acc));
+  Tensor gx = need_input_grad ? empty_in(input.sizes(), input, layout) : Tensor();
   c10::cuda::CUDAGuard guard(dev);
   mc_desc fs;
   const bool folded = weighted_folds(ds, iw, &fs);  // weighted map with plans (see conv_backward)
@@ -631,25 +651,33 @@ std::vector<Tensor> tconv_backward(const Tensor& grad_output_in, const Tensor& s
     // tensor-core path: input gradient = forward of the equivalent convolution applied to
     // grad_output; weight gradient = its weight gradient with the two tensors swapped
     Scratch ws = scratch(std::max(mc_conv_fwd_workspace_bytes(&dsu), mc_conv_wgrad_workspace_bytes(&ds)), dev);
-    check(mc_conv_fwd_tap(&dsu, grad_output.data_ptr(), tab.data_ptr(), weight.data_ptr(), nullptr,
-                          gx.data_ptr(), ws.p, ws.n, cur_stream()));
-    int rc = mc_conv_wgrad_tap(&dsu, input.data_ptr(), grad_output.data_ptr(), tab.data_ptr(),
-                               gw.data_ptr(), nullptr, cur_stream());
+    if (need_input_grad)
+      check(mc_conv_fwd_tap(&dsu, grad_output.data_ptr(), tab.data_ptr(), weight.data_ptr(), nullptr,
+                            gx.data_ptr(), ws.p, ws.n, cur_stream()));
+    if (!need_weight_grad) return {gx, Tensor(), Tensor()};
+    ParamGrads pg(weight, Cout);
+    int rc = mc_conv_wgrad_tap(&dsu, input.data_ptr(), grad_output.data_ptr(), tab.data_ptr(), pg.pw, nullptr,
+                               cur_stream());
     if (rc == MC_ERR_UNSUPPORTED)
       rc = mc_conv_wgrad(&ds, input.data_ptr(), grad_output.data_ptr(), sample_map.data_ptr(),
-                         ptr(iw), gw.data_ptr(), nullptr, ws.p, ws.n, cur_stream());
+                         ptr(iw), pg.pw, nullptr, ws.p, ws.n, cur_stream());
     check(rc);
     const mc_desc db = make_desc(input.scalar_type(), layout, B, Cout, Cout, OHt, OWt, OHt, OWt, 1, 0,
                                  interp);
-    check(mc_bias_grad(&db, grad_output.data_ptr(), gb.data_ptr(), cur_stream()));
-    return {gx, gw.to(weight.scalar_type()), gb.to(bias.scalar_type())};
+    check(mc_bias_grad(&db, grad_output.data_ptr(), pg.pb, cur_stream()));
+    pg.finish();
+    return {gx, pg.gw, pg.gb};
   }
   Scratch ws = scratch(mc_tconv_workspace_bytes(&d), dev);
-  check(mc_tconv_dgrad(&d, grad_output.data_ptr(), sample_map.data_ptr(), ptr(iw), weight.data_ptr(),
-                       gx.data_ptr(), ws.p, ws.n, cur_stream()));
+  if (need_input_grad)
+    check(mc_tconv_dgrad(&d, grad_output.data_ptr(), sample_map.data_ptr(), ptr(iw), weight.data_ptr(),
+                         gx.data_ptr(), ws.p, ws.n, cur_stream()));
+  if (!need_weight_grad) return {gx, Tensor(), Tensor()};
+  ParamGrads pg(weight, Cout);
   check(mc_tconv_wgrad(&d, grad_output.data_ptr(), input.data_ptr(), sample_map.data_ptr(), ptr(iw),
-                       gw.data_ptr(), gb.data_ptr(), ws.p, ws.n, cur_stream()));
-  return {gx, gw.to(weight.scalar_type()), gb.to(bias.scalar_type())};
+                       pg.pw, pg.pb, ws.p, ws.n, cur_stream()));
+  pg.finish();
+  return {gx, pg.gw, pg.gb};
 }
 
 // ---- pooling ----------------------------------------------------------------------------------------------
@@ -849,6 +877,127 @@ Tensor voting_resample_to_map(const Tensor& input_in, const Tensor& map_in, int6
   return out;
 }
 
+// ---- differentiable layer calls --------------------------------------------------------------------------
+// The pairing of forward and backward ops is the reference's (package/layers/nn/*.py): convolution <-> (input,
+// weight, bias gradient); max pool <-> max unpool through the stored tap offsets; average pool <-> average
+// unpool; Resample (scatter) <-> Unresample (gather).  As C++ nodes they need no interpreter: a Python
+// autograd.Function costs 8 us forward and 15-25 us backward per call (the backward thread has to take
+// the interpreter lock), which is most of the time of a small layer.  Calls that record nothing skip the node.
+using torch::autograd::AutogradContext;
+using torch::autograd::variable_list;
+
+bool records(std::initializer_list<const Tensor*> ts) {
+  if (!at::GradMode::is_enabled()) return false;
+  for (const Tensor* t : ts)
+    if (t->defined() && t->requires_grad()) return true;
+  return false;
+}
+OptTensor as_opt(const Tensor& t) { return t.defined() ? OptTensor(t) : OptTensor(); }
+Tensor or_undef(const OptTensor& t) { return t.has_value() ? *t : Tensor(); }
+
+struct ConvFn : torch::autograd::Function<ConvFn> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& w, const Tensor& b, const Tensor& map,
+                        const OptTensor& iw, int64_t K, int64_t interp, bool relu) {
+    Tensor y = conv_forward(x, map, iw, w, b, K, interp, false, relu);
+    ctx->save_for_backward({x, w, b, map, or_undef(iw), relu ? y : Tensor()});
+    ctx->saved_data["k"] = K;
+    ctx->saved_data["i"] = interp;
+    return y;
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list g) {
+    const auto s = ctx->get_saved_variables();
+    const bool need_x = ctx->needs_input_grad(0), need_p = ctx->needs_input_grad(1) || ctx->needs_input_grad(2);
+    variable_list out(8);
+    if (!need_x && !need_p) return out;
+    // (the op masks grad_output itself behind a fused ReLU: y > 0 <=> pre-activation > 0)
+    auto r = conv_backward(g[0], s[3], as_opt(s[4]), s[0], s[1], s[2], ctx->saved_data["k"].toInt(),
+                           ctx->saved_data["i"].toInt(), need_x, false, need_p, as_opt(s[5]));
+    for (int i = 0; i < 3; ++i) out[i] = r[i];
+    return out;
+  }
+};
+
+struct TconvFn : torch::autograd::Function<TconvFn> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& w, const Tensor& b, const Tensor& map,
+                        const OptTensor& iw, int64_t oh, int64_t ow, int64_t K, int64_t interp) {
+    ctx->save_for_backward({x, w, b, map, or_undef(iw)});
+    ctx->saved_data["k"] = K;
+    ctx->saved_data["i"] = interp;
+    return tconv_forward(x, map, iw, w, b, oh, ow, K, interp);
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list g) {
+    const auto s = ctx->get_saved_variables();
+    const bool need_x = ctx->needs_input_grad(0), need_p = ctx->needs_input_grad(1) || ctx->needs_input_grad(2);
+    variable_list out(9);
+    if (!need_x && !need_p) return out;
+    auto r = tconv_backward(g[0], s[3], as_opt(s[4]), s[0], s[1], s[2], ctx->saved_data["k"].toInt(),
+                            ctx->saved_data["i"].toInt(), false, need_x, need_p);
+    for (int i = 0; i < 3; ++i) out[i] = r[i];
+    return out;
+  }
+};
+
+struct MaxPoolFn : torch::autograd::Function<MaxPoolFn> {
+  static variable_list forward(AutogradContext* ctx, const Tensor& x, const Tensor& map, const OptTensor& iw, int64_t K,
+                               int64_t interp) {
+    auto r = max_pool(x, map, iw, K, interp);
+    ctx->mark_non_differentiable({r[1]});
+    ctx->set_materialize_grads(false);  // (a zero gradient for the int64 offsets would be written out otherwise)
+    ctx->save_for_backward({r[1], map, or_undef(iw)});
+    ctx->saved_data["k"] = K;
+    ctx->saved_data["i"] = interp;
+    ctx->saved_data["h"] = x.size(2);
+    ctx->saved_data["w"] = x.size(3);
+    return {r[0], r[1]};
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list g) {
+    variable_list out(5);
+    if (!g[0].defined()) return out;
+    const auto s = ctx->get_saved_variables();
+    out[0] = max_unpool(g[0], s[0], s[1], as_opt(s[2]), ctx->saved_data["h"].toInt(), ctx->saved_data["w"].toInt(),
+                        ctx->saved_data["k"].toInt(), ctx->saved_data["i"].toInt());
+    return out;
+  }
+};
+
+// Linear maps of x alone: average pool, average unpool, resample gather and scatter; the backward op of each is
+// another one of the four.  op: 0 average pool, 1 average unpool, 2 scatter, 3 gather.
+Tensor run_linear(int64_t op, const Tensor& x, const Tensor& map, const OptTensor& iw, int64_t oh, int64_t ow, int64_t K,
+                  int64_t interp) {
+  switch (op) {
+    case 0: return avg_pool(x, map, iw, K, interp);
+    case 1: return avg_unpool(x, map, iw, oh, ow, K, interp);
+    case 2: return resample_to(x, map, iw, oh, ow, interp);
+    default: return resample_from(x, map, iw, interp);
+  }
+}
+struct LinearFn : torch::autograd::Function<LinearFn> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& map, const OptTensor& iw, int64_t op,
+                        int64_t oh, int64_t ow, int64_t K, int64_t interp) {
+    ctx->save_for_backward({map, or_undef(iw)});
+    ctx->saved_data["o"] = op ^ 1;
+    ctx->saved_data["k"] = K;
+    ctx->saved_data["i"] = interp;
+    ctx->saved_data["h"] = x.size(2);
+    ctx->saved_data["w"] = x.size(3);
+    return run_linear(op, x, map, iw, oh, ow, K, interp);
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list g) {
+    const auto s = ctx->get_saved_variables();
+    variable_list out(8);
+    // (upstream gradients come in any layout; the ops want one of the two)
+    const Tensor gy = g[0].is_contiguous() || g[0].is_contiguous(at::MemoryFormat::ChannelsLast) ? g[0] : g[0].contiguous();
+    out[0] = run_linear(ctx->saved_data["o"].toInt(), gy, s[0], as_opt(s[1]), ctx->saved_data["h"].toInt(),
+                        ctx->saved_data["w"].toInt(), ctx->saved_data["k"].toInt(), ctx->saved_data["i"].toInt());
+    return out;
+  }
+};
+Tensor linear_layer(int64_t op, const Tensor& x, const Tensor& map, const OptTensor& iw, int64_t oh, int64_t ow,
+                    int64_t K, int64_t interp) {
+  if (!records({&x})) return run_linear(op, x, map, iw, oh, ow, K, interp);
+  return LinearFn::apply(x, map, iw, op, oh, ow, K, interp);
+}
+
 }  // namespace
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
@@ -950,6 +1099,33 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("cube2rect", &cube2rect);
   // VotingResampleToMap, include/nn/layers/voting_resample_layer.h:34-58
   m.def("voting_resample_to_map", &voting_resample_to_map);
+  // differentiable calls of the layer API
+  m.def("conv_layer", [](const Tensor& x, const Tensor& w, const Tensor& b, const Tensor& map, int64_t k, int64_t i,
+                         const OptTensor& iw, bool relu) {
+    if (!records({&x, &w, &b})) return conv_forward(x, map, iw, w, b, k, i, false, relu);
+    return ConvFn::apply(x, w, b, map, iw, k, i, relu);
+  });
+  m.def("tconv_layer", [](const Tensor& x, const Tensor& w, const Tensor& b, const Tensor& map, int64_t oh, int64_t ow,
+                          int64_t k, int64_t i, const OptTensor& iw) {
+    if (!records({&x, &w, &b})) return tconv_forward(x, map, iw, w, b, oh, ow, k, i);
+    return TconvFn::apply(x, w, b, map, iw, oh, ow, k, i);
+  });
+  m.def("max_pool_layer", [](const Tensor& x, const Tensor& map, int64_t k, int64_t i, const OptTensor& iw) {
+    auto r = records({&x}) ? MaxPoolFn::apply(x, map, iw, k, i) : max_pool(x, map, iw, k, i);
+    return std::make_tuple(r[0], r[1]);
+  });
+  m.def("avg_pool_layer", [](const Tensor& x, const Tensor& map, int64_t k, int64_t i, const OptTensor& iw) {
+    return linear_layer(0, x, map, iw, 0, 0, k, i);
+  });
+  m.def("avg_unpool_layer", [](const Tensor& x, int64_t oh, int64_t ow, const Tensor& map, int64_t k, int64_t i,
+                               const OptTensor& iw) { return linear_layer(1, x, map, iw, oh, ow, k, i); });
+  m.def("resample_layer", [](const Tensor& x, const Tensor& map, std::pair<int64_t, int64_t> shape, int64_t i,
+                             const OptTensor& iw) {
+    return linear_layer(2, x, map, iw, shape.first, shape.second, 1, i);
+  });
+  m.def("unresample_layer", [](const Tensor& x, const Tensor& map, int64_t i, const OptTensor& iw) {
+    return linear_layer(3, x, map, iw, 0, 0, 1, i);
+  });
   m.def("clear_plan_cache", &clear_plan_cache);
   m.def("plan_cache_kinds", &plan_cache_kinds);
   // Row plans (the fast path for maps that are translation invariant along image rows) on / off;

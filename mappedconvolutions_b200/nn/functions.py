@@ -1,4 +1,7 @@
-"""autograd.Function wrappers: each op's backward is another op of the same library.
+"""Differentiable layer calls: each op's backward is another op of the same library.
+
+With the compiled extension the calls are its C++ autograd nodes; the autograd.Function classes here
+do the same on the ctypes twin, which has none.
 
 Pairing follows the reference's package/layers/nn/*.py: conv fwd <-> (dgrad, wgrad, dbias);
 max pool <-> max unpool through the stored tap offsets; avg pool <-> avg unpool;
@@ -7,7 +10,6 @@ Resample (scatter) <-> Unresample (gather).
 import torch
 from torch.autograd import Function
 
-from ..host import COMPILED as FUSED_RELU  # the compiled extension takes relu=True
 from ..host import impl as ops
 
 
@@ -23,9 +25,6 @@ class MappedConvFn(Function):
                                                  ctx.k, ctx.interp)
             if relu:
                 y = torch.relu_(y)
-        elif relu and FUSED_RELU:
-            # the activation runs in the convolution's epilogue: no separate pass over y
-            y = ops.mapped_conv_forward(x, sample_map, weight, bias, ctx.k, ctx.interp, relu=True)
         else:
             y = ops.mapped_conv_forward(x, sample_map, weight, bias, ctx.k, ctx.interp)
             if relu:
@@ -190,3 +189,12 @@ class UnresampleFn(Function):
         else:
             gx = ops.resample_to_map(gy, sample_map, ctx.hw[0], ctx.hw[1], ctx.interp)
         return gx, None, None, None
+
+
+if hasattr(ops, "conv_layer"):  # (an extension left over from an older build has no such nodes)
+    conv, tconv, max_pool, avg_pool = ops.conv_layer, ops.tconv_layer, ops.max_pool_layer, ops.avg_pool_layer
+    avg_unpool, resample, unresample = ops.avg_unpool_layer, ops.resample_layer, ops.unresample_layer
+else:
+    conv, max_pool, avg_pool = MappedConvFn.apply, MappedMaxPoolFn.apply, MappedAvgPoolFn.apply
+    tconv = MappedTransposedConvFn.apply
+    avg_unpool, resample, unresample = MappedAvgUnpoolFn.apply, ResampleFn.apply, UnresampleFn.apply

@@ -54,8 +54,9 @@ class MappedConvolution(_ConvBase):
 
     def forward(self, x, sample_map, interp_weights=None):
         check_args(x, sample_map, interp_weights, self.in_channels, self.kernel_size)
-        return F.MappedConvFn.apply(x, self.weight, self.bias, sample_map, self.kernel_size,
-                                    self.interp, interp_weights, self.activation == 'relu')
+        p = self._parameters
+        return F.conv(x, p['weight'], p['bias'], sample_map, self.kernel_size, self.interp, interp_weights,
+                      self.activation == 'relu')
 
 
 class MappedTransposedConvolution(_ConvBase):
@@ -72,8 +73,8 @@ class MappedTransposedConvolution(_ConvBase):
     def forward(self, x, oh, ow, sample_map, interp_weights=None):
         check_args(x, sample_map, interp_weights, self.in_channels, self.kernel_size)
         check_input_map_shape(x, sample_map)
-        return F.MappedTransposedConvFn.apply(x, self.weight, self.bias, sample_map, oh, ow,
-                                              self.kernel_size, self.interp, interp_weights)
+        p = self._parameters
+        return F.tconv(x, p['weight'], p['bias'], sample_map, oh, ow, self.kernel_size, self.interp, interp_weights)
 
 
 class _PoolBase(nn.Module):
@@ -92,8 +93,7 @@ class MappedMaxPool(_PoolBase):
 
     def forward(self, x, sample_map, interp_weights=None):
         check_args(x, sample_map, interp_weights, None, self.kernel_size)
-        y, idx = F.MappedMaxPoolFn.apply(x, sample_map, self.kernel_size, self.interp,
-                                         interp_weights)
+        y, idx = F.max_pool(x, sample_map, self.kernel_size, self.interp, interp_weights)
         return (y, idx) if self.return_indices else y
 
 
@@ -105,8 +105,7 @@ class MappedAvgPool(_PoolBase):
 
     def forward(self, x, sample_map, interp_weights=None):
         check_args(x, sample_map, interp_weights, None, self.kernel_size)
-        return F.MappedAvgPoolFn.apply(x, sample_map, self.kernel_size, self.interp,
-                                       interp_weights)
+        return F.avg_pool(x, sample_map, self.kernel_size, self.interp, interp_weights)
 
 
 class MappedAvgUnpool(_PoolBase):
@@ -118,8 +117,7 @@ class MappedAvgUnpool(_PoolBase):
     def forward(self, x, oh, ow, sample_map, interp_weights=None):
         check_args(x, sample_map, interp_weights, None, self.kernel_size)
         check_input_map_shape(x, sample_map)
-        return F.MappedAvgUnpoolFn.apply(x, oh, ow, sample_map, self.kernel_size, self.interp,
-                                         interp_weights)
+        return F.avg_unpool(x, oh, ow, sample_map, self.kernel_size, self.interp, interp_weights)
 
 
 class Resample(nn.Module):
@@ -134,7 +132,7 @@ class Resample(nn.Module):
     def forward(self, x, sample_map, output_shape, interp_weights=None):
         check_args(x, sample_map, interp_weights, None, None)
         check_input_map_shape(x, sample_map)
-        return F.ResampleFn.apply(x, sample_map, output_shape, self.interp, interp_weights)
+        return F.resample(x, sample_map, output_shape, self.interp, interp_weights)
 
 
 class Unresample(nn.Module):
@@ -148,7 +146,7 @@ class Unresample(nn.Module):
 
     def forward(self, x, sample_map, interp_weights=None):
         check_args(x, sample_map, interp_weights, None, None)
-        return F.UnresampleFn.apply(x, sample_map, self.interp, interp_weights)
+        return F.unresample(x, sample_map, self.interp, interp_weights)
 
 
 def _pair(v):
