@@ -1,8 +1,8 @@
 // Generic (any dtype, any layout, weighted or not) mapped convolution kernels on the CUDA cores.
 //
-// These are the fp32 / fp64 paths (fp32 parity at 1e-5 rules out single-pass tensor-core math)
-// and the fallback for shapes the tcgen05 path does not take.  No column buffer is
-// materialised: each block interpolates a tile of the im2col matrix into shared memory and
+// These are the fp64 path and the fallback for what the tcgen05 path (bf16) and the float32 kernels
+// (conv_f32.cu: every map whose taps read at most four weighted elements) do not take.  No column
+// buffer is materialised: each block interpolates a tile of the im2col matrix into shared memory and
 // contracts it on the spot.  Row r = c_in * K + k of that matrix matches the reference's
 // include/nn/common/mapped_im2col.h:31 and weight.view(C_out, C_in*K).
 //
@@ -12,6 +12,13 @@
 #include "common.cuh"
 
 namespace mc {
+
+// conv_f32.cu
+bool conv_f32_supported(const mc_desc*);
+int conv_fwd_f32_launch(const mc_desc*, const void*, const void*, const void*, const void*, const void*, void*,
+                        cudaStream_t);
+int conv_dgrad_f32_launch(const mc_desc*, const void*, const void*, const void*, const void*, void*, cudaStream_t);
+int conv_wgrad_f32_launch(const mc_desc*, const void*, const void*, const void*, const void*, void*, cudaStream_t);
 
 struct ConvArgs {
   const void* x;    // sampled image (B, Cin, IH*IW)            [fwd, wgrad]
@@ -379,6 +386,10 @@ static ConvArgs make_args(const mc_desc* d) {
 
 int conv_fwd_simt_launch(const mc_desc* d, const void* x, const void* map, const void* iw,
                          const void* w, const void* bias, void* y, cudaStream_t st) {
+  if (conv_f32_supported(d)) {
+    const int rc = conv_fwd_f32_launch(d, x, map, iw, w, bias, y, st);
+    if (rc != MC_ERR_UNSUPPORTED) return rc;
+  }
   ConvArgs a = make_args(d);
   a.x = x; a.map = map; a.iw = d->P ? iw : nullptr; a.w = w; a.bias = bias; a.out = y;
   a.relu = (d->flags & MC_FLAG_RELU) ? 1 : 0;
@@ -406,7 +417,15 @@ int conv_dgrad_simt_launch(const mc_desc* d, const void* gy, const void* map, co
   const int fgrid = grid_for(nout, 256);
   if (d->dtype == MC_F32) {
     a.out = gx;
-    fill_bias_kernel<float, float><<<fgrid, 256, 0, st>>>((float*)gx, (const float*)bias_out, d->layout, d->C_in, a.npix_img, nout), MC_COUNT(1);
+    if (!bias_out) {
+      if (cudaMemsetAsync(gx, 0, nout * sizeof(float), st) != cudaSuccess) return MC_ERR_LAUNCH;
+    } else {
+      fill_bias_kernel<float, float><<<fgrid, 256, 0, st>>>((float*)gx, (const float*)bias_out, d->layout, d->C_in, a.npix_img, nout), MC_COUNT(1);
+    }
+    if (conv_f32_supported(d)) {
+      const int rc = conv_dgrad_f32_launch(d, gy, map, iw, w, gx, st);
+      if (rc != MC_ERR_UNSUPPORTED) return rc;
+    }
     conv_dgrad_simt<float><<<grid, 256, 0, st>>>(a), MC_COUNT(1);
   } else if (d->dtype == MC_F64) {
     a.out = gx;
@@ -468,6 +487,10 @@ int conv_wgrad_simt_launch(const mc_desc* d, const void* gy, const void* x, cons
   splits = (total_pix + a.pix_per_split - 1) / a.pix_per_split;
   const size_t esz = d->dtype == MC_F64 ? 8 : 4;
   if (cudaMemsetAsync(gw, 0, (size_t)d->C_out * a.R * esz, st) != cudaSuccess) return MC_ERR_LAUNCH;
+  if (conv_f32_supported(d)) {
+    const int rc = conv_wgrad_f32_launch(d, gy, x, map, iw, gw, st);
+    if (rc != MC_ERR_UNSUPPORTED) return rc;
+  }
   dim3 grid((unsigned)tiles, (unsigned)splits);
   if (d->dtype == MC_F32) conv_wgrad_simt<float><<<grid, 256, 0, st>>>(a), MC_COUNT(1);
   else if (d->dtype == MC_F64) conv_wgrad_simt<double><<<grid, 256, 0, st>>>(a), MC_COUNT(1);
