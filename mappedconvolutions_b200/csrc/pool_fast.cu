@@ -634,6 +634,75 @@ __global__ void __launch_bounds__(256) tap_gather_sum_kernel(const bf16* __restr
   }
 }
 
+// The same sum for maps whose lists are long (bilinear taps: about four entries per tap, 36 for 3 x 3).  Walks
+// the taps one by one: the (up to four) entries of the next tap are fetched while the rows of this tap - four
+// rows of UB images, all independent - are on their way; longer lists of a tap go on in steps of four.  The
+// entries are visited in the order of the kernel above.  Bound by the rows fetched from L2 (36 of 128 bytes per
+// pixel): 4 x 250 x 500 pixels, 64 channels, 3 x 3 bilinear taps 629 us with one row at a time beyond the twelfth
+// entry, 286 us here.
+template <int UB>
+__global__ void __launch_bounds__(256) tap_gather_sum_long_kernel(const bf16* __restrict__ z, bf16* __restrict__ out,
+                                                                  const int* __restrict__ off,
+                                                                  const int2* __restrict__ ent, int B, int C, int K,
+                                                                  long npix, long ngrid, int lpp_log2) {
+  const long gthread = blockIdx.x * 256L + threadIdx.x;
+  const long q = gthread >> lpp_log2;
+  const int c0 = (int)(gthread & ((1 << lpp_log2) - 1)) * 8;
+  if (q >= npix) return;
+  const long zrow = (long)K * C, zimg = ngrid * zrow, oimg = npix * C;
+  const int* offq = off + q * K;
+  for (int b = blockIdx.y * UB; b < B; b += UB * gridDim.y) {
+    float acc[UB][8];
+#pragma unroll
+    for (int u = 0; u < UB; ++u)
+#pragma unroll
+      for (int j = 0; j < 8; ++j) acc[u][j] = 0.f;
+    const bf16* zb = z + (long)b * zimg + c0;
+    int beg = __ldg(offq), end = __ldg(offq + 1);
+    int2 en[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) en[i] = beg + i < end ? __ldg(ent + beg + i) : make_int2(0, 0);
+    for (int k = 0; k < K;) {
+      int n = end - beg < 4 ? end - beg : 4;
+      const bf16* zk = zb + k * C;
+      uint4 r[4][UB];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int u = 0; u < UB; ++u)
+          r[i][u] = (i < n && b + u < B) ? __ldg(reinterpret_cast<const uint4*>(zk + en[i].x * zrow + u * zimg))
+                                         : make_uint4(0, 0, 0, 0);
+      float w[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) w[i] = i < n ? __int_as_float(en[i].y) : 0.f;
+      beg += n;
+      if (beg >= end) {  // on to the next tap (whose list starts where this one ended)
+        ++k;
+        if (k < K) end = __ldg(offq + k + 1);
+      }
+      if (k < K) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) en[i] = beg + i < end ? __ldg(ent + beg + i) : make_int2(0, 0);
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int u = 0; u < UB; ++u) {
+          if (i < n) {
+            float v[8];
+            Vec16<bf16>::unpack(r[i][u], v);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) acc[u][j] = fmaf(w[i], v[j], acc[u][j]);
+          }
+        }
+    }
+#pragma unroll
+    for (int u = 0; u < UB; ++u)
+      if (b + u < B)
+        *reinterpret_cast<uint4*>(out + (long)(b + u) * oimg + q * C + c0) = Vec16<bf16>::pack(acc[u]);
+  }
+}
+
 // z (B, ngrid, K * C_in) bf16, gx (B, C_in, IH, IW) channels-last bf16, inv from mc_invmap_build.
 int tap_gather_sum_launch(const mc_desc* d, const void* z, const void* inv, size_t inv_off_bytes, void* gx,
                           cudaStream_t st) {
@@ -648,9 +717,16 @@ int tap_gather_sum_launch(const mc_desc* d, const void* z, const void* inv, size
   int by = (int)((148L * 8 + xblocks - 1) / xblocks);
   if (by < 1) by = 1;
   if (by > (d->B + 1) / 2) by = (d->B + 1) / 2;
-  tap_gather_sum_kernel<<<dim3((unsigned)xblocks, (unsigned)by), 256, 0, st>>>(
-      (const bf16*)z, (bf16*)gx, (const int*)inv, (const int2*)((const uint8_t*)inv + inv_off_bytes), d->B,
-      d->C_in, d->K, npix, (long)d->OH * d->OW, lpp_log2), MC_COUNT(1);
+  const dim3 grid((unsigned)xblocks, (unsigned)by);
+  const int2* ent = (const int2*)((const uint8_t*)inv + inv_off_bytes);
+  const long ngrid = (long)d->OH * d->OW;
+  // Interpolated taps have up to four entries each; the kernel for short lists holds twelve per pixel.
+  if ((d->interp == 1 || d->interp == 2) && 4 * d->K * ngrid > 12 * npix)
+    tap_gather_sum_long_kernel<2><<<grid, 256, 0, st>>>((const bf16*)z, (bf16*)gx, (const int*)inv, ent, d->B,
+                                                        d->C_in, d->K, npix, ngrid, lpp_log2), MC_COUNT(1);
+  else
+    tap_gather_sum_kernel<<<grid, 256, 0, st>>>((const bf16*)z, (bf16*)gx, (const int*)inv, ent, d->B, d->C_in,
+                                                d->K, npix, ngrid, lpp_log2), MC_COUNT(1);
   return cudaGetLastError() == cudaSuccess ? MC_OK : MC_ERR_LAUNCH;
 }
 
