@@ -129,7 +129,10 @@ __device__ __forceinline__ CT tap_gather(const T* plane, long sp, const Tap<CT>&
   return r;
 }
 
-// Adjoint of tap_gather: plane[corner] += weight * value (atomic).
+// Adjoint of tap_gather: plane[corner] += weight * value (atomic).  A product that is exactly zero is
+// left out: the sums start at +0 or a bias and cannot be changed by it (NaN compares unequal and is
+// added).  Barycentric maps name whole vertices, so three of the four corners of each of their points
+// have weight zero.
 template <typename CT>
 __device__ __forceinline__ void tap_scatter(CT* plane, long sp, const Tap<CT>& t, CT value) {
   if (t.n == 1) {
@@ -137,8 +140,10 @@ __device__ __forceinline__ void tap_scatter(CT* plane, long sp, const Tap<CT>& t
     return;
   }
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
-    if (t.off[i] >= 0) atomicAdd(plane + (long)t.off[i] * sp, mul_rn(t.w[i], value));
+  for (int i = 0; i < 4; ++i) {
+    const CT v = mul_rn(t.w[i], value);
+    if (t.off[i] >= 0 && v != CT(0)) atomicAdd(plane + (long)t.off[i] * sp, v);
+  }
 }
 
 // Strides (in elements) of a (B, C, H*W) activation in either layout.
