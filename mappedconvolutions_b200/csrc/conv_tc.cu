@@ -23,6 +23,7 @@
 // Replaces the per-batch im2col / col2im + cublasSgemm sequences of the reference's
 // src/nn/cuda/mapped_convolution_layer.cu:39-70, :100-127, :155-190.
 #include <cub/device/device_scan.cuh>
+#include <cuda.h>  // CUtensorMap (types only: the driver entry point is looked up at run time)
 
 #include <atomic>
 #include <mutex>
@@ -319,7 +320,8 @@ __device__ __forceinline__ void issue_row(const TapEnt* ent, const bf16* sb, int
   L.v[0] = ldg16(sb + (long)(int)o.x * C);
   L.v[1] = ldg16(sb + (long)(int)o.y * C);
   L.v[2] = ldg16(sb + (long)(int)o.z * C);
-  L.v[3] = ldg16(sb + (long)o3 * C);
+  // (barycentric maps have three points: a quarter of the row fetches)
+  L.v[3] = w.w != 0u ? ldg16(sb + (long)o3 * C) : make_uint4(0, 0, 0, 0);
 }
 
 __device__ __forceinline__ void blend_row(const RowLoad& L, float2 (&acc)[4]) {
@@ -1011,6 +1013,96 @@ __device__ __forceinline__ void producer_loop_copy(const Source& s, const Tiling
   }
 }
 
+// Nearest maps with a compact table: a row of a stage is a row of the source tensor or zeros, so the TMA
+// unit can fetch it - four rows per instruction (tile::gather4; 64 channels of four arbitrary rows), already in
+// the 128-byte swizzle, rows beyond the tensor filled with zeros.  A lane owns four neighbouring rows; a warp issues
+// a whole stage, and GATHER_WARPS warps take turns, so that the table loads of one slice overlap with the issue of
+// the others.  Against the copy through registers this needs no shared-memory stores, no proxy fence per stage and
+// no tap table in shared memory, whose 57 KB (7 taps) become pipeline stages.
+constexpr int GATHER_WARPS = 4;
+__device__ __forceinline__ void tma_gather4(uint32_t dst_smem, const CUtensorMap* tm, int col, const int (&row)[4],
+                                            uint32_t bar) {
+  // (col is a multiple of 64 elements: the 16-byte rule of the innermost coordinate)
+  asm volatile(
+      "cp.async.bulk.tensor.2d.shared::cluster.global.tile::gather4.mbarrier::complete_tx::bytes [%0], "
+      "[%1, {%2, %3, %4, %5, %6}], [%7];"
+      :
+      : "r"(dst_smem), "l"((uint64_t)tm), "r"(col), "r"(row[0]), "r"(row[1]), "r"(row[2]), "r"(row[3]), "r"(bar)
+      : "memory");
+}
+
+// nslots ring slots per tile, the first nsl with data, the others zero; sl0: first slice of this CTA.
+__device__ __forceinline__ void producer_loop_gather(const Source& s, const Tiling& t, const CUtensorMap* tm, int nsl,
+                                                     int nslots, int nst, uint32_t stage0, uint32_t full0,
+                                                     uint32_t empty0, volatile int* abort_flag, int pw, int lane,
+                                                     int code, int sl0) {
+  const int cpb = s.C / 64;
+  const int none = (int)(s.src_elems / s.C);  // first row past the tensor: reads as zeros
+  // Warp pw takes the ring steps pw, pw + gw, pw + 2 gw, .. of the whole run, across tiles.  gw <= nst, and that
+  // matters: step n waits for step n - nst to be read, by the parity of its slot, which is only unambiguous once step
+  // n - 2 nst has been read - as this warp's previous step, n - gw >= n - nst, has already waited for.
+  const uint32_t gw = nst < GATHER_WARPS ? nst : GATHER_WARPS;
+  if ((uint32_t)pw >= gw) return;
+  uint32_t n0 = 0;  // ring step of the tile's first slot
+  for (int tile = blockIdx.x; tile < t.tiles; tile += gridDim.x, n0 += nslots) {
+    const int* tp[4];
+    int base[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      long gp, p;
+      int img;
+      bool valid;
+      tile_pixel(t, tile, 4 * lane + j, gp, img, p, valid);
+      tp[j] = valid ? s.tab32 + p * s.K : nullptr;
+      base[j] = (int)(img * s.spix);
+    }
+    for (int sl = (int)((pw + gw - n0 % gw) % gw); sl < nslots; sl += gw) {
+      const int e = sl0 + sl, tap = e / cpb;
+      int row[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) row[j] = tp[j] && sl < nsl ? __ldg(tp[j] + tap) : -1;
+      const uint32_t n = n0 + sl, q = n / (uint32_t)nst, st = n - q * nst;
+      int okw = 1;
+      if (lane == 0) {
+        okw = mbar_wait(empty0 + 8u * st, (q & 1) ^ 1, abort_flag, code) ? 1 : 0;
+        if (okw) mbar_expect_tx(full0 + 8u * st, STAGE_BYTES);
+      }
+      okw = __shfl_sync(0xffffffffu, okw, 0);
+      if (!okw) {  // given up: the copies still in flight land within microseconds
+        const long long c0 = clock64();
+        while (clock64() - c0 < 4000000) __nanosleep(1000);
+        return;
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) row[j] = row[j] >= 0 ? base[j] + row[j] : none;
+      tma_gather4(stage0 + st * STAGE_BYTES + lane * 512u, tm, sl < nsl ? (e - tap * cpb) * 64 : 0, row,
+                  full0 + 8u * st);
+    }
+  }
+}
+
+// Tensor map of a (rows, C) bf16 tensor for tma_gather4.
+static bool make_gather_map(CUtensorMap* tm, const void* base, long rows, int C) {
+  static std::atomic<void*> fn{nullptr};
+  void* f = fn.load(std::memory_order_acquire);
+  if (!f) {
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &q) != cudaSuccess ||
+        q != cudaDriverEntryPointSuccess || !f)
+      return false;
+    fn.store(f, std::memory_order_release);
+  }
+  using Encode = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
+                              const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
+                              CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+  const cuuint64_t dims[2] = {(cuuint64_t)C, (cuuint64_t)rows};
+  const cuuint64_t strides[1] = {(cuuint64_t)C * 2};
+  const cuuint32_t box[2] = {64, 1}, estr[2] = {1, 1};
+  return ((Encode)f)(tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
+                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 // Shared-memory carve-up common to both kernels.
 struct Smem {
   uint32_t stage0, extra0, bar0;
@@ -1054,15 +1146,22 @@ static size_t smem_bytes(int nst, size_t extra_bytes, int nfloat, int nbar) {
 // slice of every pipeline step is streamed in beside its stage by a bulk copy (needs PRE, whose
 // idle decoder warps provide the thread that issues the copies).
 // blockIdx.y selects the chunk of NOUT output channels.
-template <int NOUT, bool CSR, bool PRE, bool WRES>
-__global__ void __launch_bounds__(TC_THREADS, 1) conv_gemm_tc_kernel(const GemmArgs a) {
+// The kernel may start while the weight image is still being written (launch_gemm_kernel): everything
+// else it reads was complete before that kernel began, and whoever reads the image waits for it here.
+__device__ __forceinline__ void weights_ready() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// TMA: the rows are fetched by producer_loop_gather and there is no tap table in shared memory.
+template <int NOUT, bool CSR, bool PRE, bool WRES, bool TMA>
+__global__ void __launch_bounds__(TC_THREADS, 1) conv_gemm_tc_kernel(const GemmArgs a,
+                                                                  const __grid_constant__ CUtensorMap tmap) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   const int nst = a.nst;
   const int co0 = blockIdx.y * NOUT;
   constexpr uint32_t WSLICE = NOUT * 128;  // bytes of one weight slice
   const size_t wbytes = (size_t)(WRES ? a.nsl : nst) * WSLICE;
+  const size_t tabb = TMA ? 0 : tap_table_bytes(a.s.K);
   // bars: full[nst], empty[nst], tfull[2], tempty[2], drain, tab_full[2], tab_empty[2]
-  const Smem sm = carve(smem_raw, nst, wbytes + tap_table_bytes(a.s.K) + EPI_STAGING_BYTES, NOUT,
+  const Smem sm = carve(smem_raw, nst, wbytes + tabb + EPI_STAGING_BYTES, NOUT,
                         2 * nst + 9);
   float* bias_s = sm.fl;
   volatile int* abort_flag = sm.abort_flag;
@@ -1095,6 +1194,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) conv_gemm_tc_kernel(const GemmA
   }
   // resident operands: weight slices and bias
   if (WRES) {
+    weights_ready();
     for (int i = threadIdx.x; i < a.nsl * NOUT * 8; i += TC_THREADS) {
       const int sl = i / (NOUT * 8), j = i - sl * (NOUT * 8);
       sts16(w0 + 16u * i, ldg16(a.wimg + ((size_t)sl * a.ncol + co0) * 8 + j));
@@ -1103,7 +1203,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) conv_gemm_tc_kernel(const GemmA
   for (int i = threadIdx.x; i < NOUT; i += TC_THREADS)
     bias_s[i] = a.bias && co0 + i < a.ocol ? __bfloat162float(a.bias[co0 + i]) : 0.f;
   fence_proxy_async_smem();
-  {  // the K zero-weight entries behind the two table halves
+  if (!TMA) {  // the K zero-weight entries behind the two table halves
     uint4* z = reinterpret_cast<uint4*>((TapEnt*)(sm.extra + wbytes) + (size_t)2 * TILE_M * a.s.K);
     for (int i = threadIdx.x; i < 2 * a.s.K; i += TC_THREADS) z[i] = make_uint4(0, 0, 0, 0);
   }
@@ -1151,7 +1251,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) conv_gemm_tc_kernel(const GemmA
     // warp passes the 32 x 64-byte block through shared memory and stores 8 rows x 64 bytes per
     // instruction (lane -> row 8 i + lane / 4, 16-byte piece lane % 4).
     const int q = warp & 3;  // TMEM lane quarter this warp may read
-    const uint32_t stg = w0 + (uint32_t)(wbytes + tap_table_bytes(a.s.K)) + (uint32_t)(warp - 1) * 2048u;
+    const uint32_t stg = w0 + (uint32_t)(wbytes + tabb) + (uint32_t)(warp - 1) * 2048u;
     const uint32_t wr_row = stg + lane * 64, wr_x = (lane >> 1) & 3;
     uint32_t rd_addr[4];
 #pragma unroll
@@ -1224,12 +1324,13 @@ __global__ void __launch_bounds__(TC_THREADS, 1) conv_gemm_tc_kernel(const GemmA
     // ------------------------------------------------------------------ producers
     if (warp < FIRST_PROD_WARP) {
       if (PRE) {
-        if (warp == FIRST_DEC_WARP && lane == 0 && a.s.packed != 2)
+        if (!TMA && warp == FIRST_DEC_WARP && lane == 0 && a.s.packed != 2)
           loader_loop(a.s, a.t, w0 + (uint32_t)wbytes, tabbar0, abort_flag);
         if (!WRES && warp == FIRST_DEC_WARP + 1 && lane == 0) {
           // weight streamer: slice s of every tile goes into the ring slot of pipeline step s
           uint32_t st = 0, ph = 0;
           bool ok = true;
+          weights_ready();
           for (int tile = blockIdx.x; tile < a.t.tiles && ok; tile += gridDim.x) {
             for (int s = 0; s < a.nsl; ++s) {
               ok = mbar_wait(empty_bar(st), ph ^ 1, abort_flag, 0x73);
@@ -1244,6 +1345,10 @@ __global__ void __launch_bounds__(TC_THREADS, 1) conv_gemm_tc_kernel(const GemmA
         decoder_loop<CSR>(a.s, a.t, (TapEnt*)(sm.extra + wbytes), tabbar0, abort_flag,
                           (warp - FIRST_DEC_WARP) * 32 + lane, lane);
       }
+    } else if constexpr (TMA) {
+      if (warp < FIRST_PROD_WARP + GATHER_WARPS)
+        producer_loop_gather(a.s, a.t, &tmap, a.nsl, a.nsl, nst, stage0, full_bar(0), empty_bar(0), abort_flag,
+                             warp - FIRST_PROD_WARP, lane, 0x37, 0);
     } else if (!CSR && PRE && a.s.packed == 2) {
       producer_rowwise<false>(a.s, a.t, a.nsl, a.nsl, nst, stage0, full_bar(0), empty_bar(0),
                               (TapEnt*)(sm.extra + wbytes), abort_flag, warp - FIRST_PROD_WARP, lane,
@@ -1281,13 +1386,14 @@ __global__ void __launch_bounds__(TC_THREADS, 1) conv_gemm_tc_kernel(const GemmA
 // to gw with atomics at the end.
 constexpr int GY_STAGES = 2;
 
-template <int NOUT, bool PRE>
-__global__ void __launch_bounds__(TC_THREADS, 1) conv_wgrad_tc_kernel(const GemmArgs a) {
+template <int NOUT, bool PRE, bool TMA>
+__global__ void __launch_bounds__(TC_THREADS, 1) conv_wgrad_tc_kernel(const GemmArgs a,
+                                                                   const __grid_constant__ CUtensorMap tmap) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   const int nst = a.nst;  // even
   constexpr uint32_t GYB = (NOUT / 64) * STAGE_BYTES;  // one gy tile: 128 pixels x NOUT channels
   // bars: full[nst], empty[nst], gfull[GY], gempty[GY], done
-  const Smem sm = carve(smem_raw, nst, (size_t)GY_STAGES * GYB + tap_table_bytes(a.s.K), NOUT,
+  const Smem sm = carve(smem_raw, nst, (size_t)GY_STAGES * GYB + (TMA ? 0 : tap_table_bytes(a.s.K)), NOUT,
                         2 * nst + 2 * GY_STAGES + 5);
   float* gb_s = sm.fl;
   volatile int* abort_flag = sm.abort_flag;
@@ -1330,7 +1436,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) conv_wgrad_tc_kernel(const Gemm
     fence_barrier_init();
   }
   for (int i = threadIdx.x; i < NOUT; i += TC_THREADS) gb_s[i] = 0.f;
-  {  // the K zero-weight entries behind the two table halves
+  if (!TMA) {  // the K zero-weight entries behind the two table halves
     uint4* z = reinterpret_cast<uint4*>((TapEnt*)(sm.extra + (size_t)GY_STAGES * GYB) +
                                         (size_t)2 * TILE_M * a.s.K);
     for (int i = threadIdx.x; i < 2 * a.s.K; i += TC_THREADS) z[i] = make_uint4(0, 0, 0, 0);
@@ -1389,8 +1495,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) conv_wgrad_tc_kernel(const Gemm
       okw = __shfl_sync(0xffffffffu, okw, 0);
       if (!okw) { ok = false; break; }
       const uint32_t sbase = gy0 + gs * GYB;
-      if (nsl_pad <= 2 || (a.s.interp == 0 && a.s.C <= 64)) {
-        // Few, cheap slices per tile (one-slice layers, 64-channel copies): the gy tile's load
+      if (nsl_pad <= 2 || (a.s.interp == 0 && a.s.C <= 64) || TMA) {
+        // Few, cheap slices per tile (one-slice layers, 64-channel copies, TMA gathers): the gy tile's load
         // latency is on the critical path, so all eight rows of a group are requested before the
         // first is stored.
 #pragma unroll
@@ -1483,12 +1589,16 @@ __global__ void __launch_bounds__(TC_THREADS, 1) conv_wgrad_tc_kernel(const Gemm
     // ------------------------------------------------------------------ producers
     if (warp < FIRST_PROD_WARP) {
       if (PRE) {
-        if (warp == FIRST_DEC_WARP && lane == 0 && a.s.packed != 2)
+        if (!TMA && warp == FIRST_DEC_WARP && lane == 0 && a.s.packed != 2)
           loader_loop(a.s, a.t, gy0 + (uint32_t)GY_STAGES * GYB, tabbar0, abort_flag);
       } else {
         decoder_loop<false>(a.s, a.t, (TapEnt*)(sm.extra + (size_t)GY_STAGES * GYB), tabbar0,
                             abort_flag, (warp - FIRST_DEC_WARP) * 32 + lane, lane);
       }
+    } else if constexpr (TMA) {
+      if (warp < FIRST_PROD_WARP + GATHER_WARPS)
+        producer_loop_gather(a.s, a.t, &tmap, nsl, nsl_pad, nst, stage0, full_bar(0), empty_bar(0), abort_flag,
+                             warp - FIRST_PROD_WARP, lane, 0x65, sl0);
     } else if (PRE && a.s.packed == 2) {
       producer_rowwise<true>(a.s, a.t, nsl, nsl_pad, nst, stage0, full_bar(0), empty_bar(0),
                              (TapEnt*)(sm.extra + (size_t)GY_STAGES * GYB), abort_flag,
@@ -1532,6 +1642,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) conv_wgrad_tc_kernel(const Gemm
 // `rows` real rows of `rows_img` (a multiple of 64); the others are zero.
 __global__ void weight_image_kernel(const bf16* __restrict__ w, uint16_t* __restrict__ img, int rows,
                                     int rows_img, int red, int K, int transpose, int Cin_w) {
+  asm volatile("griddepcontrol.launch_dependents;");  // the GEMM's blocks may start setting up
   const int nsl = (K * red + 63) / 64;
   const long total = (long)nsl * rows_img * 64;
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < total;
@@ -1755,24 +1866,48 @@ struct GemmPlan {
   size_t extra;  // shared memory behind the stages: weights + tap table
 };
 
-static bool plan_gemm(int ncol, int nsl, int K, GemmPlan& p) {
+// tabb: bytes of the tap table in shared memory
+static bool plan_gemm_tab(int ncol, int nsl, size_t tabb, GemmPlan& p) {
   if (ncol <= 0 || ncol % 64 != 0) return false;
   // resident weights when they fit with a reasonable pipeline (needs ncol <= 256)
   if (ncol <= 256 && (ncol == 64 || ncol == 128 || ncol == 256)) {
-    const size_t extra = (size_t)nsl * ncol * 128 + tap_table_bytes(K) + EPI_STAGING_BYTES;
+    const size_t extra = (size_t)nsl * ncol * 128 + tabb + EPI_STAGING_BYTES;
     const int nst = pick_stages(extra, ncol, 8, 3, false);
     if (nst > 0) { p = {ncol, true, nst, extra}; return true; }
   }
   const int nout = ncol % 256 == 0 ? 256 : ncol % 128 == 0 ? 128 : 64;
   // streamed weights: every stage carries its weight slice
   for (int nst = 6; nst >= 3; --nst) {
-    const size_t extra = (size_t)nst * nout * 128 + tap_table_bytes(K) + EPI_STAGING_BYTES;
+    const size_t extra = (size_t)nst * nout * 128 + tabb + EPI_STAGING_BYTES;
     if (smem_bytes(nst, extra, nout, 2 * nst + 16) <= SMEM_LIMIT) {
       p = {nout, false, nst, extra};
       return true;
     }
   }
   return false;
+}
+
+static bool plan_gemm(int ncol, int nsl, int K, GemmPlan& p) {
+  return plan_gemm_tab(ncol, nsl, tap_table_bytes(K), p);
+}
+
+// The plan for `tiles` pixel tiles with a prebuilt tap table.  Where tiles x column chunks do not fill half of
+// the SMs, narrower chunks put the idle ones to work: each gathers the same rows again, but streams and
+// multiplies a half or a quarter of the weights.  Blocks that see a single tile stream their weights, which overlaps
+// with the gathers, instead of waiting for all of them first.
+static bool plan_gemm_tiles(int ncol, int nsl, size_t tabb, long tiles, GemmPlan& p) {
+  if (!plan_gemm_tab(ncol, nsl, tabb, p)) return false;
+  int nout = p.nout;
+  while (nout > 64 && 2 * tiles * (ncol / nout) <= sm_count()) nout /= 2;
+  if (nout == p.nout && (!p.wres || nsl == 1 || tiles * (ncol / nout) > sm_count())) return true;
+  for (int nst = 8; nst >= 3; --nst) {
+    const size_t extra = (size_t)nst * nout * 128 + tabb + EPI_STAGING_BYTES;
+    if (smem_bytes(nst, extra, nout, 2 * nst + 16) <= SMEM_LIMIT) {
+      p = {nout, false, nst, extra};
+      break;
+    }
+  }
+  return true;
 }
 
 // 64-element slices of the gathered (tap, input channel) axis of forward / wgrad
@@ -1813,38 +1948,63 @@ size_t conv_tc_fwd_ws(const mc_desc* d) {
   return conv_tc_fwd_wimg_bytes(d) + (fwd_needs_table(d) ? tapmap_bytes(d) : 0);
 }
 
+// Directly behind weight_image_kernel: the launch may overlap with it (only the weights are waited for).  Done
+// where every block works on at most two tiles: there the few microseconds count (encoder of four layers on
+// 10 242 vertices, batch 1, with the narrower column chunks of plan_gemm_tiles: 106 -> 77 us), while long launches
+// measured 0.5 - 1 % slower with it.
+static bool short_launch(long tiles, int chunks) { return tiles * chunks <= 2L * sm_count(); }
+
+template <typename Kern>
+static int launch_gemm_kernel(Kern kern, dim3 grid, size_t smem, cudaStream_t st, const GemmArgs& a,
+                              const CUtensorMap& tm, bool overlap) {
+  if (!allow_big_smem(kern)) return MC_ERR_LAUNCH;
+  cudaLaunchAttribute attr = {};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(TC_THREADS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = &attr;
+  cfg.numAttrs = overlap ? 1 : 0;
+  if (cudaLaunchKernelEx(&cfg, kern, a, tm) != cudaSuccess) return MC_ERR_LAUNCH;
+  MC_COUNT(1);
+  return MC_OK;
+}
+
 template <int NOUT, bool CSR>
-static int launch_gemm_n(const GemmArgs& a, const GemmPlan& p, bool pre, cudaStream_t st) {
+static int launch_gemm_n(const GemmArgs& a, const CUtensorMap* tma, const GemmPlan& p, bool pre, bool overlap,
+                         cudaStream_t st) {
   const size_t smem = smem_bytes(a.nst, p.extra, NOUT, 2 * a.nst + 9);
   const int ny = a.ncol / NOUT;
   int gx = sm_count() / ny;
   if (gx < 1) gx = 1;
   if (gx > a.t.tiles) gx = a.t.tiles;
   const dim3 grid(gx, ny);
-  if (p.wres) {
-    if (pre) {
-      if (!allow_big_smem(conv_gemm_tc_kernel<NOUT, CSR, true, true>)) return MC_ERR_LAUNCH;
-      conv_gemm_tc_kernel<NOUT, CSR, true, true><<<grid, TC_THREADS, smem, st>>>(a), MC_COUNT(1);
-    } else {
-      if (CSR) return MC_ERR_UNSUPPORTED;
-      if (!allow_big_smem(conv_gemm_tc_kernel<NOUT, false, false, true>)) return MC_ERR_LAUNCH;
-      conv_gemm_tc_kernel<NOUT, false, false, true><<<grid, TC_THREADS, smem, st>>>(a), MC_COUNT(1);
-    }
-  } else {
-    if (!pre) return MC_ERR_UNSUPPORTED;
-    if (!allow_big_smem(conv_gemm_tc_kernel<NOUT, CSR, true, false>)) return MC_ERR_LAUNCH;
-    conv_gemm_tc_kernel<NOUT, CSR, true, false><<<grid, TC_THREADS, smem, st>>>(a), MC_COUNT(1);
+  const CUtensorMap none = {};
+  int rc = MC_ERR_UNSUPPORTED;
+  if constexpr (!CSR) {
+    if (p.wres && !pre) rc = launch_gemm_kernel(conv_gemm_tc_kernel<NOUT, false, false, true, false>, grid, smem, st, a, none, overlap);
   }
+  if constexpr (!CSR) {
+    if (tma && p.wres) rc = launch_gemm_kernel(conv_gemm_tc_kernel<NOUT, false, true, true, true>, grid, smem, st, a, *tma, overlap);
+    if (tma && !p.wres) rc = launch_gemm_kernel(conv_gemm_tc_kernel<NOUT, false, true, false, true>, grid, smem, st, a, *tma, overlap);
+  }
+  if (!tma && p.wres && pre) rc = launch_gemm_kernel(conv_gemm_tc_kernel<NOUT, CSR, true, true, false>, grid, smem, st, a, none, overlap);
+  if (!tma && !p.wres && pre) rc = launch_gemm_kernel(conv_gemm_tc_kernel<NOUT, CSR, true, false, false>, grid, smem, st, a, none, overlap);
+  if (rc) return rc;
   MC_CHECK_LAUNCH();
   return MC_OK;
 }
 
 template <bool CSR>
-static int launch_gemm(const GemmArgs& a, const GemmPlan& p, bool pre, cudaStream_t st) {
+static int launch_gemm(const GemmArgs& a, const CUtensorMap* tma, const GemmPlan& p, bool pre, bool overlap,
+                       cudaStream_t st) {
   switch (p.nout) {
-    case 64: return launch_gemm_n<64, CSR>(a, p, pre, st);
-    case 128: return launch_gemm_n<128, CSR>(a, p, pre, st);
-    case 256: return launch_gemm_n<256, CSR>(a, p, pre, st);
+    case 64: return launch_gemm_n<64, CSR>(a, tma, p, pre, overlap, st);
+    case 128: return launch_gemm_n<128, CSR>(a, tma, p, pre, overlap, st);
+    case 256: return launch_gemm_n<256, CSR>(a, tma, p, pre, overlap, st);
   }
   return MC_ERR_UNSUPPORTED;
 }
@@ -1898,6 +2058,12 @@ int tapmap_build_weighted_launch(const mc_desc* d, const void* map, const void* 
 }
 
 // map != null: the kernel decodes the map itself; tab != null: prebuilt table (tapmap_build_launch)
+// The producer for nearest maps that lets the TMA unit fetch the rows: whole 64-channel blocks, a prebuilt table.
+static bool gather_by_tma(const mc_desc* d, const void* x, const void* tab, CUtensorMap* tm) {
+  return d->interp == 0 && d->C_in % 64 == 0 && tapmap_compact(d, tab) &&
+         make_gather_map(tm, x, (long)d->B * d->IH * d->IW, d->C_in);
+}
+
 static int fwd_launch_impl(const mc_desc* d, const void* x, const void* map, const void* tab,
                            const void* w, const void* bias, void* y, void* ws, size_t ws_bytes,
                            cudaStream_t st) {
@@ -1921,7 +2087,12 @@ static int fwd_launch_impl(const mc_desc* d, const void* x, const void* map, con
   a.ncol = pad64(d->C_out);
   a.relu = (d->flags & MC_FLAG_RELU) ? 1 : 0;
   GemmPlan p;
-  if (!plan_gemm(a.ncol, a.nsl, d->K, p)) return MC_ERR_UNSUPPORTED;
+  // (a raw map builds its table, if at all, for the plan that knows no tile count)
+  CUtensorMap tm = {};
+  const bool tma = gather_by_tma(d, x, tab, &tm);
+  const size_t tabb = tma ? 0 : tap_table_bytes(d->K);
+  if (!(tab ? plan_gemm_tiles(a.ncol, a.nsl, tabb, a.t.tiles, p) : plan_gemm(a.ncol, a.nsl, d->K, p)))
+    return MC_ERR_UNSUPPORTED;
   a.nst = p.nst;
   const long nw = (long)a.nsl * 64 * a.ncol;
   weight_image_kernel<<<grid_for(nw, 256), 256, 0, st>>>((const bf16*)w, (uint16_t*)ws, d->C_out, a.ncol,
@@ -1938,7 +2109,12 @@ static int fwd_launch_impl(const mc_desc* d, const void* x, const void* map, con
     a.full_cnt = N_PRODUCER_WARPS / ROW_TEAMS;
     a.s.tab32 = tapmap_compact(d, a.s.tab);
   }
-  return launch_gemm<false>(a, p, a.s.tab != nullptr, st);
+  if (tma) {
+    a.full_cnt = 1;
+    a.s.tab32 = tapmap_compact(d, tab);
+  }
+  return launch_gemm<false>(a, tma ? &tm : nullptr, p, a.s.tab != nullptr,
+                            tab != nullptr && short_launch(a.t.tiles, a.ncol / p.nout), st);
 }
 
 int conv_tc_fwd_launch(const mc_desc* d, const void* x, const void* map, const void* w,
@@ -2066,13 +2242,13 @@ int conv_tc_dgrad_launch(const mc_desc* d, const void* gy, const void* inv, cons
   a.ncol = pad64(d->C_in);
   a.relu = (bias_out && (d->flags & MC_FLAG_RELU)) ? 1 : 0;  // the transposed layer's forward
   GemmPlan p;
-  if (!plan_gemm(a.ncol, a.nsl, d->K, p)) return MC_ERR_UNSUPPORTED;
+  if (!plan_gemm_tiles(a.ncol, a.nsl, tap_table_bytes(d->K), a.t.tiles, p)) return MC_ERR_UNSUPPORTED;
   a.nst = p.nst;
   a.full_cnt = N_PRODUCER_WARPS;
   const long nw = (long)a.nsl * 64 * a.ncol;
   weight_image_kernel<<<grid_for(nw, 256), 256, 0, st>>>((const bf16*)w, (uint16_t*)ws, d->C_in, a.ncol,
                                                          d->C_out, d->K, 1, d->C_in), MC_COUNT(1);
-  return launch_gemm<true>(a, p, true, st);
+  return launch_gemm<true>(a, nullptr, p, true, short_launch(a.t.tiles, a.ncol / p.nout), st);
 }
 
 // ---- wgrad -----------------------------------------------------------------------------------------------
@@ -2085,7 +2261,7 @@ struct WgradPlan {
   size_t extra;
 };
 
-static bool plan_wgrad(const mc_desc* d, WgradPlan& p) {
+static bool plan_wgrad(const mc_desc* d, size_t tabb, WgradPlan& p) {
   if (d->C_out % 8 != 0 || (long)d->K * d->C_in >= (1L << 24)) return false;
   const int nsl = fwd_slices(d);
   const int nmt = (nsl + 1) / 2;
@@ -2094,7 +2270,7 @@ static bool plan_wgrad(const mc_desc* d, WgradPlan& p) {
   const int cap = 512 / p.nout;
   p.groups = (nmt + cap - 1) / cap;
   p.mtpg = (nmt + p.groups - 1) / p.groups;
-  p.extra = (size_t)GY_STAGES * (p.nout / 64) * STAGE_BYTES + tap_table_bytes(d->K);
+  p.extra = (size_t)GY_STAGES * (p.nout / 64) * STAGE_BYTES + tabb;
   p.nst = pick_stages(p.extra, p.nout, 10, 4, true);
   return p.nst > 0;
 }
@@ -2102,22 +2278,26 @@ static bool plan_wgrad(const mc_desc* d, WgradPlan& p) {
 bool conv_tc_wgrad_supported(const mc_desc* d) {
   if (d->dtype != MC_BF16 || d->layout != MC_NHWC || d->P != 0) return false;
   WgradPlan p;
-  return plan_wgrad(d, p);
+  return plan_wgrad(d, tap_table_bytes(d->K), p);
 }
 size_t conv_tc_wgrad_ws(const mc_desc*) { return 0; }
 
 template <int NOUT>
-static int launch_wgrad_n(const GemmArgs& a, const WgradPlan& p, bool pre, cudaStream_t st) {
+static int launch_wgrad_n(const GemmArgs& a, const CUtensorMap* tma, const WgradPlan& p, bool pre, cudaStream_t st) {
   const size_t smem = smem_bytes(a.nst, p.extra, NOUT, 2 * a.nst + 2 * GY_STAGES + 5);
   int gx = sm_count() / (p.groups * p.chunks);
   if (gx < 1) gx = 1;
   if (gx > a.t.tiles) gx = a.t.tiles;
   const dim3 grid(gx, p.groups, p.chunks);
-  if (!allow_big_smem(conv_wgrad_tc_kernel<NOUT, false>) ||
-      !allow_big_smem(conv_wgrad_tc_kernel<NOUT, true>))
+  auto run = [&](auto kern, const CUtensorMap& tm) {
+    if (!allow_big_smem(kern)) return false;
+    kern<<<grid, TC_THREADS, smem, st>>>(a, tm), MC_COUNT(1);
+    return true;
+  };
+  if (!(tma ? run(conv_wgrad_tc_kernel<NOUT, true, true>, *tma)
+            : pre ? run(conv_wgrad_tc_kernel<NOUT, true, false>, CUtensorMap{})
+                  : run(conv_wgrad_tc_kernel<NOUT, false, false>, CUtensorMap{})))
     return MC_ERR_LAUNCH;
-  if (pre) conv_wgrad_tc_kernel<NOUT, true><<<grid, TC_THREADS, smem, st>>>(a), MC_COUNT(1);
-  else conv_wgrad_tc_kernel<NOUT, false><<<grid, TC_THREADS, smem, st>>>(a), MC_COUNT(1);
   MC_CHECK_LAUNCH();
   return MC_OK;
 }
@@ -2147,13 +2327,20 @@ static int wgrad_launch_impl(const mc_desc* d, const void* gy, const void* x, co
   a.ocol = d->C_out;
   a.ncol = pad64(d->C_out);
   WgradPlan p;
-  if (!plan_wgrad(d, p)) return MC_ERR_UNSUPPORTED;
+  CUtensorMap tm = {};
+  const bool tma = gather_by_tma(d, x, tab, &tm);
+  const size_t tabb = tma ? 0 : tap_table_bytes(d->K);
+  if (!plan_wgrad(d, tabb, p)) return MC_ERR_UNSUPPORTED;
   a.nst = p.nst;
   a.mtpg = p.mtpg;
   a.full_cnt = N_PRODUCER_WARPS;
   if (tab && rowwise_shape(d) && p.nst >= ROW_TEAMS) {
     a.s.packed = 2;
     a.full_cnt = N_PRODUCER_WARPS / ROW_TEAMS;
+    a.s.tab32 = tapmap_compact(d, tab);
+  }
+  if (tma) {
+    a.full_cnt = 1;
     a.s.tab32 = tapmap_compact(d, tab);
   }
   const size_t nw = (size_t)d->C_out * d->C_in * d->K;
@@ -2164,8 +2351,8 @@ static int wgrad_launch_impl(const mc_desc* d, const void* gy, const void* x, co
   // very few input channels and a nearest map with its compact table: one pass over grad_output
   if (tab && smallcin_wgrad_shape(d) && tapmap_compact(d, tab))
     return smallcin_wgrad_launch(d, gy, ymask, x, tapmap_compact(d, tab), gw, gb, st);
-  return p.nout == 128 ? launch_wgrad_n<128>(a, p, tab != nullptr, st)
-                       : launch_wgrad_n<64>(a, p, tab != nullptr, st);
+  return p.nout == 128 ? launch_wgrad_n<128>(a, tma ? &tm : nullptr, p, tab != nullptr, st)
+                       : launch_wgrad_n<64>(a, tma ? &tm : nullptr, p, tab != nullptr, st);
 }
 
 int conv_tc_wgrad_launch(const mc_desc* d, const void* gy, const void* x, const void* map, void* gw,
