@@ -247,10 +247,10 @@ static int launch_fwd(const mc_desc* d, const void* x, const void* map, const vo
 // The image side is zeroed and scattered into in chunks of whole planes / images that stay in L2: over the
 // whole tensor at once every atomic read-modify-write would fetch a line that the memset had already pushed out
 // to HBM.  Each launch clears the target of the next one.  bf16: the sums of a chunk are rounded into the result
-// before the next chunk reuses their buffer.  Max unpooling of 32 x 128 planes of 163 842 vertices: 2.18 ms with one
-// memset and one scatter, 1.85 ms in chunks of 16 MB (8 MB: 2.2, 32 MB: 1.9, 64 MB: 2.7); what is left is the rate of
-// scattered atomics in L2, about 86 per ns.
-constexpr long SCATTER_CHUNK_BYTES = 16L << 20;
+// before the next chunk reuses their buffer.  Max pooling and unpooling of 32 x 128 planes of 163 842 vertices: 3.47 ms
+// with one memset and one scatter, 3.14 ms in chunks of 32 MB (16 MB: 3.45, 64 MB: 3.97); what is left of the scatter
+// (1.85 of 2.18 ms) is the rate of scattered atomics in L2, about 86 per ns.
+constexpr long SCATTER_CHUNK_BYTES = 32L << 20;
 
 template <typename T, int OP>
 static int launch_bwd_chunks(ScatterArgs a, typename Traits<T>::CT* acc, bf16* rounded, cudaStream_t st) {
