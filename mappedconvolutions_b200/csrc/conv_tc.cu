@@ -1948,12 +1948,9 @@ size_t conv_tc_fwd_ws(const mc_desc* d) {
   return conv_tc_fwd_wimg_bytes(d) + (fwd_needs_table(d) ? tapmap_bytes(d) : 0);
 }
 
-// Directly behind weight_image_kernel: the launch may overlap with it (only the weights are waited for).  Done
-// where every block works on at most two tiles: there the few microseconds count (encoder of four layers on
-// 10 242 vertices, batch 1, with the narrower column chunks of plan_gemm_tiles: 106 -> 77 us), while long launches
-// measured 0.5 - 1 % slower with it.
-static bool short_launch(long tiles, int chunks) { return tiles * chunks <= 2L * sm_count(); }
-
+// Directly behind weight_image_kernel: the launch may overlap with it (only the weights are waited for).  Encoder of
+// four layers on 10 242 vertices, batch 1, together with the narrower column chunks of plan_gemm_tiles: 106 -> 77 us;
+// 64 -> 64 barycentric layer on 8 x 40 962 vertices: 646 us without, 632 us with it.
 template <typename Kern>
 static int launch_gemm_kernel(Kern kern, dim3 grid, size_t smem, cudaStream_t st, const GemmArgs& a,
                               const CUtensorMap& tm, bool overlap) {
@@ -2114,7 +2111,7 @@ static int fwd_launch_impl(const mc_desc* d, const void* x, const void* map, con
     a.s.tab32 = tapmap_compact(d, tab);
   }
   return launch_gemm<false>(a, tma ? &tm : nullptr, p, a.s.tab != nullptr,
-                            tab != nullptr && short_launch(a.t.tiles, a.ncol / p.nout), st);
+                            tab != nullptr, st);
 }
 
 int conv_tc_fwd_launch(const mc_desc* d, const void* x, const void* map, const void* w,
@@ -2248,7 +2245,7 @@ int conv_tc_dgrad_launch(const mc_desc* d, const void* gy, const void* inv, cons
   const long nw = (long)a.nsl * 64 * a.ncol;
   weight_image_kernel<<<grid_for(nw, 256), 256, 0, st>>>((const bf16*)w, (uint16_t*)ws, d->C_in, a.ncol,
                                                          d->C_out, d->K, 1, d->C_in), MC_COUNT(1);
-  return launch_gemm<true>(a, nullptr, p, true, short_launch(a.t.tiles, a.ncol / p.nout), st);
+  return launch_gemm<true>(a, nullptr, p, true, true, st);
 }
 
 // ---- wgrad -----------------------------------------------------------------------------------------------
