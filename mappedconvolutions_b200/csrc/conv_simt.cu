@@ -299,10 +299,30 @@ __global__ void __launch_bounds__(256) bias_grad_kernel(const T* gy, CT* gb, int
   long end = beg + pix_per_split;
   if (end > total) end = total;
   CT s = CT(0);
-  for (long g = beg + threadIdx.x; g < end; g += 256) {
-    const int b = (int)(g / npix);
-    const long p = g % npix;
-    s += (CT)ldv(gy + b * gs.b + c * gs.c + p * gs.p);
+  if (npix >= 1024) {
+    // image by image: no division per value, eight loads in flight (64 channels of 4 x 128 x 256
+    // float32 pixels: 21.6 -> 7.8 us)
+    for (long g = beg; g < end;) {
+      const long b = g / npix, p0 = g - b * npix;
+      const long n = npix - p0 < end - g ? npix - p0 : end - g;
+      const T* src = gy + b * gs.b + c * gs.c + p0 * gs.p;
+      CT part[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) part[j] = CT(0);
+      long i = threadIdx.x;
+      for (; i + 7 * 256 < n; i += 8 * 256)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) part[j] += (CT)ldv(src + (i + j * 256) * gs.p);
+      for (; i < n; i += 256) part[0] += (CT)ldv(src + i * gs.p);
+      s += ((part[0] + part[1]) + (part[2] + part[3])) + ((part[4] + part[5]) + (part[6] + part[7]));
+      g += n;
+    }
+  } else {
+    for (long g = beg + threadIdx.x; g < end; g += 256) {
+      const int b = (int)(g / npix);
+      const long p = g % npix;
+      s += (CT)ldv(gy + b * gs.b + c * gs.c + p * gs.p);
+    }
   }
   __shared__ CT red[256];
   red[threadIdx.x] = s;
