@@ -320,8 +320,9 @@ __device__ __forceinline__ void issue_row(const TapEnt* ent, const bf16* sb, int
   L.v[0] = ldg16(sb + (long)(int)o.x * C);
   L.v[1] = ldg16(sb + (long)(int)o.y * C);
   L.v[2] = ldg16(sb + (long)(int)o.z * C);
-  // (barycentric maps have three points: a quarter of the row fetches)
-  L.v[3] = w.w != 0u ? ldg16(sb + (long)o3 * C) : make_uint4(0, 0, 0, 0);
+  // (fetched unconditionally: a predicate on its weight costs more than the row - barycentric layer 628 -> 636 us,
+  // bilinear 1281 -> 1316 us)
+  L.v[3] = ldg16(sb + (long)o3 * C);
 }
 
 __device__ __forceinline__ void blend_row(const RowLoad& L, float2 (&acc)[4]) {
@@ -1950,7 +1951,7 @@ size_t conv_tc_fwd_ws(const mc_desc* d) {
 
 // Directly behind weight_image_kernel: the launch may overlap with it (only the weights are waited for).  Encoder of
 // four layers on 10 242 vertices, batch 1, together with the narrower column chunks of plan_gemm_tiles: 106 -> 77 us;
-// 64 -> 64 barycentric layer on 8 x 40 962 vertices: 646 us without, 632 us with it.
+// 64 -> 64 barycentric layer on 8 x 40 962 vertices, training step: 646 us without, 641 us with it.
 template <typename Kern>
 static int launch_gemm_kernel(Kern kern, dim3 grid, size_t smem, cudaStream_t st, const GemmArgs& a,
                               const CUtensorMap& tm, bool overlap) {
