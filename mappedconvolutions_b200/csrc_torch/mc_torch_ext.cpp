@@ -12,6 +12,7 @@
 // mappedconvolutions_b200/ops.py is the same host logic on ctypes; the tests use it to reach the
 // C ABI without a compiler, and check the two against each other.
 #include <algorithm>
+#include <torch/csrc/jit/frontend/tracer.h>
 #include <torch/extension.h>
 
 #include <c10/cuda/CUDAGuard.h>
@@ -886,6 +887,19 @@ Tensor voting_resample_to_map(const Tensor& input_in, const Tensor& map_in, int6
 using torch::autograd::AutogradContext;
 using torch::autograd::variable_list;
 
+// Calls that somebody records or transforms: under a tracer the graph would hold the allocation of the output
+// and not the kernel that fills it; a forward-mode tangent would be dropped without a word; a functorch
+// transform would meet raw pointers.  The layer calls below return None for them, and the caller takes the
+// Python autograd.Function (recorded as one op, refused by the other two).
+bool seen_by_torch(std::initializer_list<const Tensor*> ts) {
+  if (torch::jit::tracer::isTracing() ||
+      c10::impl::tls_is_dispatch_key_included(c10::DispatchKey::FuncTorchDynamicLayerFrontMode))
+    return true;
+  for (const Tensor* t : ts)
+    if (t && t->defined() && t->_fw_grad(/*level=*/0).defined()) return true;
+  return false;
+}
+
 bool records(std::initializer_list<const Tensor*> ts) {
   if (!at::GradMode::is_enabled()) return false;
   for (const Tensor* t : ts)
@@ -992,8 +1006,9 @@ struct LinearFn : torch::autograd::Function<LinearFn> {
     return out;
   }
 };
-Tensor linear_layer(int64_t op, const Tensor& x, const Tensor& map, const OptTensor& iw, int64_t oh, int64_t ow,
-                    int64_t K, int64_t interp) {
+OptTensor linear_layer(int64_t op, const Tensor& x, const Tensor& map, const OptTensor& iw, int64_t oh, int64_t ow,
+                       int64_t K, int64_t interp) {
+  if (seen_by_torch({&x, &map, opt(iw)})) return c10::nullopt;
   if (!records({&x})) return run_linear(op, x, map, iw, oh, ow, K, interp);
   return LinearFn::apply(x, map, iw, op, oh, ow, K, interp);
 }
@@ -1099,18 +1114,22 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("cube2rect", &cube2rect);
   // VotingResampleToMap, include/nn/layers/voting_resample_layer.h:34-58
   m.def("voting_resample_to_map", &voting_resample_to_map);
-  // differentiable calls of the layer API
+  // differentiable calls of the layer API (None: see seen_by_torch)
   m.def("conv_layer", [](const Tensor& x, const Tensor& w, const Tensor& b, const Tensor& map, int64_t k, int64_t i,
-                         const OptTensor& iw, bool relu) {
+                         const OptTensor& iw, bool relu) -> OptTensor {
+    if (seen_by_torch({&x, &w, &b, &map, opt(iw)})) return c10::nullopt;
     if (!records({&x, &w, &b})) return conv_forward(x, map, iw, w, b, k, i, false, relu);
     return ConvFn::apply(x, w, b, map, iw, k, i, relu);
   });
   m.def("tconv_layer", [](const Tensor& x, const Tensor& w, const Tensor& b, const Tensor& map, int64_t oh, int64_t ow,
-                          int64_t k, int64_t i, const OptTensor& iw) {
+                          int64_t k, int64_t i, const OptTensor& iw) -> OptTensor {
+    if (seen_by_torch({&x, &w, &b, &map, opt(iw)})) return c10::nullopt;
     if (!records({&x, &w, &b})) return tconv_forward(x, map, iw, w, b, oh, ow, k, i);
     return TconvFn::apply(x, w, b, map, iw, oh, ow, k, i);
   });
-  m.def("max_pool_layer", [](const Tensor& x, const Tensor& map, int64_t k, int64_t i, const OptTensor& iw) {
+  m.def("max_pool_layer", [](const Tensor& x, const Tensor& map, int64_t k, int64_t i,
+                             const OptTensor& iw) -> c10::optional<std::tuple<Tensor, Tensor>> {
+    if (seen_by_torch({&x, &map, opt(iw)})) return c10::nullopt;
     auto r = records({&x}) ? MaxPoolFn::apply(x, map, iw, k, i) : max_pool(x, map, iw, k, i);
     return std::make_tuple(r[0], r[1]);
   });

@@ -1,7 +1,9 @@
 """Differentiable layer calls: each op's backward is another op of the same library.
 
-With the compiled extension the calls are its C++ autograd nodes; the autograd.Function classes here
-do the same on the ctypes twin, which has none.
+With the compiled extension the calls are its C++ autograd nodes.  The autograd.Function classes here do the
+same on the ctypes twin, which has none, and where torch has to see the call as one Python function: a tracer
+would only record the allocation of the C++ call's output, a forward-mode tangent would be dropped without a
+word, and a functorch transform expects the refusal that an autograd.Function gives.
 
 Pairing follows the reference's package/layers/nn/*.py: conv fwd <-> (dgrad, wgrad, dbias);
 max pool <-> max unpool through the stored tap offsets; avg pool <-> avg unpool;
@@ -191,10 +193,22 @@ class UnresampleFn(Function):
         return gx, None, None, None
 
 
-if hasattr(ops, "conv_layer"):  # (an extension left over from an older build has no such nodes)
-    conv, tconv, max_pool, avg_pool = ops.conv_layer, ops.tconv_layer, ops.max_pool_layer, ops.avg_pool_layer
-    avg_unpool, resample, unresample = ops.avg_unpool_layer, ops.resample_layer, ops.unresample_layer
-else:
-    conv, max_pool, avg_pool = MappedConvFn.apply, MappedMaxPoolFn.apply, MappedAvgPoolFn.apply
-    tconv = MappedTransposedConvFn.apply
-    avg_unpool, resample, unresample = MappedAvgUnpoolFn.apply, ResampleFn.apply, UnresampleFn.apply
+def _layer_call(function, node_name):
+    """The extension's node of that name, which returns None where torch has to see the Function (see above)."""
+    node = getattr(ops, node_name, None)  # (the ctypes twin has no nodes)
+    if node is None:
+        return function.apply
+
+    def call(*args):
+        out = node(*args)
+        return function.apply(*args) if out is None else out
+    return call
+
+
+conv = _layer_call(MappedConvFn, "conv_layer")
+tconv = _layer_call(MappedTransposedConvFn, "tconv_layer")
+max_pool = _layer_call(MappedMaxPoolFn, "max_pool_layer")
+avg_pool = _layer_call(MappedAvgPoolFn, "avg_pool_layer")
+avg_unpool = _layer_call(MappedAvgUnpoolFn, "avg_unpool_layer")
+resample = _layer_call(ResampleFn, "resample_layer")
+unresample = _layer_call(UnresampleFn, "unresample_layer")
