@@ -54,8 +54,7 @@ class MappedConvolution(_ConvBase):
 
     def forward(self, x, sample_map, interp_weights=None):
         check_args(x, sample_map, interp_weights, self.in_channels, self.kernel_size)
-        p = self._parameters
-        return F.conv(x, p['weight'], p['bias'], sample_map, self.kernel_size, self.interp, interp_weights,
+        return F.conv(x, self.weight, self.bias, sample_map, self.kernel_size, self.interp, interp_weights,
                       self.activation == 'relu')
 
 
@@ -73,8 +72,7 @@ class MappedTransposedConvolution(_ConvBase):
     def forward(self, x, oh, ow, sample_map, interp_weights=None):
         check_args(x, sample_map, interp_weights, self.in_channels, self.kernel_size)
         check_input_map_shape(x, sample_map)
-        p = self._parameters
-        return F.tconv(x, p['weight'], p['bias'], sample_map, oh, ow, self.kernel_size, self.interp, interp_weights)
+        return F.tconv(x, self.weight, self.bias, sample_map, oh, ow, self.kernel_size, self.interp, interp_weights)
 
 
 class _PoolBase(nn.Module):

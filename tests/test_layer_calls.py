@@ -104,3 +104,43 @@ def test_functorch_transforms_are_refused(calls, make, m):
         with pytest.raises(RuntimeError, match="functorch transforms"):
             f()
     assert not calls
+
+
+def _layer_and_args(transposed):
+    if transposed:
+        return mnn.MappedTransposedConvolution(4, 3, 5), (torch.zeros(1, 4, 6, 7), 8, 9, torch.zeros(6, 7, 5, 2))
+    return mnn.MappedConvolution(4, 3, 5), (torch.zeros(1, 4, 6, 7), torch.zeros(6, 7, 5, 2))
+
+
+def _prune(layer):
+    import torch.nn.utils.prune as prune
+    prune.random_unstructured(layer, "weight", amount=0.3)
+
+
+def _shared_memory_copy(layer):
+    replica = layer._replicate_for_data_parallel()  # (what nn.DataParallel calls: parameters become plain attributes)
+    for name, p in layer.named_parameters():
+        setattr(replica, name, p.clone())
+    return replica
+
+
+@pytest.mark.filterwarnings("ignore::FutureWarning")
+@pytest.mark.parametrize("transposed", [False, True])
+@pytest.mark.parametrize("change", [
+    lambda l: None, torch.nn.utils.parametrizations.weight_norm, torch.nn.utils.parametrizations.spectral_norm,
+    torch.nn.utils.weight_norm, torch.nn.utils.spectral_norm, _prune, _shared_memory_copy,
+], ids=["plain", "weight_norm", "spectral_norm", "old weight_norm", "old spectral_norm", "prune", "data parallel"])
+def test_parameters_that_are_attributes_only(monkeypatch, transposed, change):
+    layer, args = _layer_and_args(transposed)
+    layer = change(layer) or layer
+    seen = {}
+
+    def op(x, weight, bias, *rest):
+        seen.update(weight=weight, bias=bias)
+        return (weight.sum() + bias.sum()).reshape(1, 1, 1, 1)
+
+    monkeypatch.setattr(F, "tconv" if transposed else "conv", op)
+    layer(*args).sum().backward()
+    assert seen["weight"].shape == ((4, 3, 5) if transposed else (3, 4, 5)) and seen["bias"].shape == (3,)
+    if "_shared" not in change.__name__:
+        assert all(p.grad is not None for p in layer.parameters())
