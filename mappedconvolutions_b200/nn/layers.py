@@ -91,7 +91,7 @@ class MappedMaxPool(_PoolBase):
 
     def forward(self, x, sample_map, interp_weights=None):
         check_args(x, sample_map, interp_weights, None, self.kernel_size)
-        y, idx = F.max_pool(x, sample_map, self.kernel_size, self.interp, interp_weights)
+        y, idx = F.max_pool(x, sample_map, int(self.kernel_size), self.interp, interp_weights)
         return (y, idx) if self.return_indices else y
 
 
@@ -103,7 +103,7 @@ class MappedAvgPool(_PoolBase):
 
     def forward(self, x, sample_map, interp_weights=None):
         check_args(x, sample_map, interp_weights, None, self.kernel_size)
-        return F.avg_pool(x, sample_map, self.kernel_size, self.interp, interp_weights)
+        return F.avg_pool(x, sample_map, int(self.kernel_size), self.interp, interp_weights)
 
 
 class MappedAvgUnpool(_PoolBase):
@@ -115,7 +115,7 @@ class MappedAvgUnpool(_PoolBase):
     def forward(self, x, oh, ow, sample_map, interp_weights=None):
         check_args(x, sample_map, interp_weights, None, self.kernel_size)
         check_input_map_shape(x, sample_map)
-        return F.avg_unpool(x, oh, ow, sample_map, self.kernel_size, self.interp, interp_weights)
+        return F.avg_unpool(x, oh, ow, sample_map, int(self.kernel_size), self.interp, interp_weights)
 
 
 class Resample(nn.Module):
@@ -130,7 +130,7 @@ class Resample(nn.Module):
     def forward(self, x, sample_map, output_shape, interp_weights=None):
         check_args(x, sample_map, interp_weights, None, None)
         check_input_map_shape(x, sample_map)
-        return F.resample(x, sample_map, output_shape, self.interp, interp_weights)
+        return F.resample(x, sample_map, (int(output_shape[0]), int(output_shape[1])), self.interp, interp_weights)
 
 
 class Unresample(nn.Module):

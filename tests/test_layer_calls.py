@@ -144,3 +144,15 @@ def test_parameters_that_are_attributes_only(monkeypatch, transposed, change):
     assert seen["weight"].shape == ((4, 3, 5) if transposed else (3, 4, 5)) and seen["bias"].shape == (3,)
     if "_shared" not in change.__name__:
         assert all(p.grad is not None for p in layer.parameters())
+
+
+@pytest.mark.parametrize("call", [
+    lambda x, m: mnn.Resample()(x, m[:, :, 0], (8.0, 9.0)),              # H / 2, a numpy or tensor size
+    lambda x, m: mnn.Resample()(x, m[:, :, 0], (8, 9, 3)),               # an image's shape
+    lambda x, m: mnn.Resample()(x, m[:, :, 0], torch.tensor([8.0, 9.0])),
+    lambda x, m: mnn.MappedMaxPool(5.0)(x, m), lambda x, m: mnn.MappedAvgPool(5.0)(x, m),
+    lambda x, m: mnn.MappedAvgUnpool(5.0)(x, 8, 9, m),
+])
+def test_sizes_are_converted_to_whole_numbers(call):
+    with pytest.raises(RuntimeError, match="CUDA only"):  # (the op took the call; there is no CPU path)
+        call(torch.zeros(1, 2, 4, 6), torch.zeros(4, 6, 5, 2))
