@@ -120,9 +120,12 @@ struct Source {
   const int* tab32;     // nearest maps: the same table as one int per entry (source pixel or -1)
   long src_elems;       // elements of src (batch * spix * C)
   int KC;      // K * C: length of the gathered (tap, channel) axis
-  int packed;  // C is not a multiple of 64: a 64-wide slice holds elements tap * C + c of several
-               // taps (map mode only).  2: the whole axis fits one slice and the row-per-thread
+  int packed;  // a 64-wide slice holds elements tap * C + c of several taps (C is not a multiple of 64, or
+               // split).  2: the whole axis fits one slice and the row-per-thread
                // producer builds it straight from the global tap table
+  int exact;   // padded output columns: corners of weight zero are left out (packed producer)
+  int split;   // 1: every slice takes two ring slots, the float32 values rounded to bf16 and what the rounding
+               // left of them (packed producer): about 16 significant bits instead of 8
 };
 
 // Replace the inactive corners of a decoded tap by (some active pixel of the tap, weight 0).
@@ -347,6 +350,33 @@ __device__ __forceinline__ uint4 pack_row(const float2 (&acc)[4]) {
   return o;
 }
 
+// What rounding to bf16 left of two values; nothing beyond the largest finite one (inf - inf is no number).
+__device__ __forceinline__ uint32_t pack_rest2(float2 v, uint32_t rounded) {
+  const float h0 = __uint_as_float(rounded << 16), h1 = __uint_as_float(rounded & 0xFFFF0000u);
+  return pack_bf16x2(fabsf(h0) < INFINITY ? v.x - h0 : 0.f, fabsf(h1) < INFINITY ? v.y - h1 : 0.f);
+}
+__device__ __forceinline__ uint4 pack_rest(const float2 (&acc)[4], const uint4& rounded) {
+  return make_uint4(pack_rest2(acc[0], rounded.x), pack_rest2(acc[1], rounded.y), pack_rest2(acc[2], rounded.z),
+                    pack_rest2(acc[3], rounded.w));
+}
+
+// Entries 4 and up of the inverse-map list `key`, added to the float32 sums of its first four.
+__device__ __forceinline__ void add_list_rest(const int* __restrict__ inv_off, const int2* __restrict__ inv_ent, int C,
+                                              long key, const bf16* base, float2 (&acc)[4]) {
+  const int end = __ldg(inv_off + key + 1);
+#pragma unroll 1
+  for (int e = __ldg(inv_off + key) + 4; e < end; ++e) {
+    const int2 en = __ldg(inv_ent + e);
+    const uint4 v = ldg16(base + (long)en.x * C);
+    const float w = __int_as_float(en.y);
+    const float2 w2 = make_float2(w, w);
+    ffma2_bf16x2(acc[0], w2, v.x);
+    ffma2_bf16x2(acc[1], w2, v.y);
+    ffma2_bf16x2(acc[2], w2, v.z);
+    ffma2_bf16x2(acc[3], w2, v.w);
+  }
+}
+
 // Inverse-map mode, rare (0.5 % of the lists of a gnomonic 3x3 map): entries `first` and up of the
 // list `key` = (input pixel, tap).  Runs after the row has been written: it re-reads the bf16 row
 // from the stage, adds the remaining terms and writes it back, so that the hot loop keeps no state
@@ -519,35 +549,65 @@ __device__ __forceinline__ void producer_loop_map(const Source& s, const Tiling&
   }
 }
 
-// Producer warp for channel counts that are not a multiple of 64 (inverse-map mode: a multiple of 8).  The gathered axis is
+// Producer warp for channel counts that are not a multiple of 64, and for split rows.  The gathered axis is
 // e = tap * C + c, cut into 64-element slices and zero-padded at the end; a lane owns 8 consecutive
 // elements of a row.  With C % 8 == 0 those lie in one tap and are fetched as 16-byte vectors like
 // in the regular producer, only with a tap of the lane's own; otherwise (e.g. the 3 input channels
 // of a first layer) every element is gathered on its own.
+// EXACT (layers with padded output columns, and all of the inverse-map mode): corners of weight zero are not read,
+// so that an infinity or NaN only reaches the outputs that use it, as it does on the CUDA cores; and rows may be
+// split - nsl, nslots and sl0 count ring slots, of which a slice then takes two.  Against rows that are rounded once
+// this costs, on 4 x 200 x 400 pixels with 9 bilinear taps, 32 -> 32 channels: forward 105 -> 142 us, input gradient
+// 135 -> 170 us, weight gradient 138 -> 194 us; 128 -> 96: 295 -> 492, 348 -> 449, 422 -> 641 us (CUDA cores: 1.3 ms
+// and more for 32 -> 32, 14.5 ms and more for 128 -> 96).
+template <bool EXACT>
 __device__ __forceinline__ float gather_element(const TapEnt* ent, const bf16* sb, int C, int c) {
   float acc = 0.f;
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const int off = i == 3 ? (ent->off[3] & ~MORE_FLAG) : ent->off[i];
-    const float v = __bfloat162float(__ldg(sb + (long)off * C + c));
-    acc = fmaf(ent->w[i], v, acc);
+    const float w = ent->w[i], v = __bfloat162float(__ldg(sb + (long)off * C + c));
+    acc = fmaf(w, EXACT && w == 0.f ? 0.f : v, acc);
   }
   return acc;
 }
 
-__device__ __forceinline__ uint4 gather_elements8(const TapEnt* trow, const bf16* sb, int C, int KC,
-                                                  int e0) {
-  float v[8];
+template <bool EXACT>
+__device__ __forceinline__ void gather_elements8(const TapEnt* trow, const bf16* sb, int C, int KC, int e0,
+                                                 float2 (&acc)[4]) {
   int k = e0 / C, c = e0 - k * C;
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
-    v[j] = e0 + j < KC ? gather_element(trow + k, sb, C, c) : 0.f;
+    const float v = e0 + j < KC ? gather_element<EXACT>(trow + k, sb, C, c) : 0.f;
+    if (j & 1) acc[j / 2].y = v; else acc[j / 2].x = v;
     if (++c == C) { c = 0; ++k; }
   }
-  return pack8(v);
 }
 
-template <bool CSR, bool PAD>
+// zeros where on == 0
+__device__ __forceinline__ uint4 ldg16_if(const void* p, uint32_t on) {
+  uint4 v = make_uint4(0, 0, 0, 0);
+  asm volatile(
+      "{\n .reg .pred p;\n setp.ne.u32 p, %5, 0;\n @p ld.global.nc.v4.u32 {%0, %1, %2, %3}, [%4];\n}"
+      : "+r"(v.x), "+r"(v.y), "+r"(v.z), "+r"(v.w)
+      : "l"(p), "r"(on));
+  return v;
+}
+
+// issue_row without the corners of weight zero (seal_entry leaves no -0)
+__device__ __forceinline__ void issue_active(const TapEnt* ent, const bf16* sb, int C, RowLoad& L) {
+  const uint4* e = reinterpret_cast<const uint4*>(ent);
+  const uint4 o = e[0], w = e[1];
+  const uint32_t off[4] = {o.x, o.y, o.z, o.w & ~(uint32_t)MORE_FLAG}, wb[4] = {w.x, w.y, w.z, w.w};
+  L.more = (o.w & (uint32_t)MORE_FLAG) != 0;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    L.w[i] = __uint_as_float(wb[i]);
+    L.v[i] = ldg16_if(sb + (long)(int)off[i] * C, wb[i]);
+  }
+}
+
+template <bool CSR, bool PAD, bool EXACT>
 __device__ __forceinline__ void producer_loop_packed(const Source& s, const Tiling& t, int nsl,
                                                      int nslots, int nst, uint32_t stage0,
                                                      uint32_t full0, uint32_t empty0, TapEnt* table,
@@ -556,10 +616,26 @@ __device__ __forceinline__ void producer_loop_packed(const Source& s, const Tili
   const int g = lane >> 3, lg = lane & 7;
   const int C = s.C, KC = s.KC;
   const bool vec = (C & 7) == 0;
+  const int split = EXACT ? s.split : 0;
   const int r0 = pw * 4 + g, r1 = r0 + N_PRODUCER_WARPS * 4;
   const uint32_t so0 = r0 * 128 + ((lg ^ (r0 & 7)) << 4), so1 = r1 * 128 + ((lg ^ (r1 & 7)) << 4);
   const uint4 zero = make_uint4(0, 0, 0, 0);
   uint32_t st = 0, ph = 0, it = 0;
+  // two rows into the next ring slot
+  auto put = [&](const uint4& ra, const uint4& rb) {
+    int okw = 1;
+    if (lane == 0) okw = mbar_wait(empty0 + 8u * st, ph ^ 1, abort_flag, code) ? 1 : 0;
+    okw = __shfl_sync(0xffffffffu, okw, 0);
+    if (!okw) return false;
+    const uint32_t sbase = stage0 + st * STAGE_BYTES;
+    sts16(sbase + so0, ra);
+    sts16(sbase + so1, rb);
+    fence_proxy_async_smem();
+    __syncwarp();
+    if (lane == 0) mbar_arrive(full0 + 8u * st);
+    if (++st == (uint32_t)nst) { st = 0; ph ^= 1; }
+    return true;
+  };
   for (int tile = blockIdx.x; tile < t.tiles; tile += gridDim.x, ++it) {
     const TapEnt* tab = table + (size_t)(it & 1) * TILE_M * s.K;
     {
@@ -582,45 +658,35 @@ __device__ __forceinline__ void producer_loop_packed(const Source& s, const Tili
       if (g1 < t.mtot) s1 = s.src + (g1 / t.npix) * s.spix * C; else t1 = zero_ent;
     }
     const int p0 = CSR ? tile_row_pixel(t, tile, r0) : 0, p1 = CSR ? tile_row_pixel(t, tile, r1) : 0;
-    int e0 = sl0 * 64 + lg * 8;
-    for (int sl = 0; sl < nslots; ++sl, e0 += 64) {
+    int e0 = (sl0 >> split) * 64 + lg * 8;
+    for (int sl = 0; sl < nslots; sl += 1 + split, e0 += 64) {
       const bool live = (!PAD || sl < nsl) && e0 < KC;
-      uint4 ra = zero, rb = zero;
-      bool more_a = false, more_b = false;
-      int tap_k = 0, tap_c = 0;
+      float2 va[4], vb[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) va[j] = vb[j] = make_float2(0.f, 0.f);
       if (live) {
         if (vec) {
           const int k = e0 / C, c = e0 - k * C;
           RowLoad A, B;
-          issue_row<CSR>(t0 + k, s0 + c, C, A);
-          issue_row<CSR>(t1 + k, s1 + c, C, B);
-          float2 acc[4];
-          blend_row(A, acc);
-          ra = pack_row(acc);
-          blend_row(B, acc);
-          rb = pack_row(acc);
-          more_a = CSR && A.more; more_b = CSR && B.more;
-          tap_k = k; tap_c = c;
+          if (EXACT) {
+            issue_active(t0 + k, s0 + c, C, A);
+            issue_active(t1 + k, s1 + c, C, B);
+          } else {
+            issue_row<CSR>(t0 + k, s0 + c, C, A);
+            issue_row<CSR>(t1 + k, s1 + c, C, B);
+          }
+          blend_row(A, va);
+          blend_row(B, vb);
+          if (CSR && A.more) add_list_rest(s.inv_off, s.inv_ent, C, (long)p0 * s.K + k, s0 + c, va);
+          if (CSR && B.more) add_list_rest(s.inv_off, s.inv_ent, C, (long)p1 * s.K + k, s1 + c, vb);
         } else {
-          ra = gather_elements8(t0, s0, C, KC, e0);
-          rb = gather_elements8(t1, s1, C, KC, e0);
+          gather_elements8<EXACT>(t0, s0, C, KC, e0, va);
+          gather_elements8<EXACT>(t1, s1, C, KC, e0, vb);
         }
       }
-      int okw = 1;
-      if (lane == 0) okw = mbar_wait(empty0 + 8u * st, ph ^ 1, abort_flag, code) ? 1 : 0;
-      okw = __shfl_sync(0xffffffffu, okw, 0);
-      if (!okw) return;
-      const uint32_t sbase = stage0 + st * STAGE_BYTES;
-      sts16(sbase + so0, ra);
-      sts16(sbase + so1, rb);
-      if (CSR) {
-        if (more_a) add_list_tail(s.inv_off, s.inv_ent, C, (long)p0 * s.K + tap_k, s0 + tap_c, sbase + so0, 4);
-        if (more_b) add_list_tail(s.inv_off, s.inv_ent, C, (long)p1 * s.K + tap_k, s1 + tap_c, sbase + so1, 4);
-      }
-      fence_proxy_async_smem();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(full0 + 8u * st);
-      if (++st == (uint32_t)nst) { st = 0; ph ^= 1; }
+      const uint4 ra = pack_row(va), rb = pack_row(vb);
+      if (!put(ra, rb)) return;
+      if (EXACT && split && !put(pack_rest(va, ra), pack_rest(vb, rb))) return;
     }
     __syncwarp();
     if (lane == 0) mbar_arrive(tabbar0 + 16 + 8 * (it & 1));
@@ -700,7 +766,7 @@ __device__ __forceinline__ void gather_row_nearest(const TapEnt* ent, const bf16
 #pragma unroll
       for (int j = 0; j < PE; ++j) {
         if (pass * PE + j < 64 && pass * PE + j < KC) {
-          v[j] = __uint_as_float(e.y) * __bfloat162float(__ldg(xb + (long)(int)e.x * C + c));
+          v[j] = e.y ? __bfloat162float(__ldg(xb + (long)(int)e.x * C + c)) : 0.f;  // (weights are 1 or 0)
           if (++c == C) {
             c = 0;
             if (++k < K) e = mine[k];
@@ -912,20 +978,7 @@ __device__ __forceinline__ uint4 finish_list(const TapEnt* ent, const bf16* sb, 
     ffma2_bf16x2(acc[2], w2, v.z);
     ffma2_bf16x2(acc[3], w2, v.w);
   }
-  if (o3 & MORE_FLAG) {
-    const int end = __ldg(inv_off + key + 1);
-#pragma unroll 1
-    for (int e = __ldg(inv_off + key) + 4; e < end; ++e) {
-      const int2 en = __ldg(inv_ent + e);
-      const uint4 v = ldg16(sb + (long)en.x * C);
-      const float w = __int_as_float(en.y);
-      const float2 w2 = make_float2(w, w);
-      ffma2_bf16x2(acc[0], w2, v.x);
-      ffma2_bf16x2(acc[1], w2, v.y);
-      ffma2_bf16x2(acc[2], w2, v.z);
-      ffma2_bf16x2(acc[3], w2, v.w);
-    }
-  }
+  if (o3 & MORE_FLAG) add_list_rest(inv_off, inv_ent, C, key, sb, acc);
   return pack_row(acc);
 }
 
@@ -1174,6 +1227,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) conv_gemm_tc_kernel(const GemmA
   auto tempty_bar = [&](int i) { return bar0 + 8u * (2 * nst + 2 + i); };
   const uint32_t drain_bar = bar0 + 8u * (2 * nst + 4);
   const uint32_t tabbar0 = bar0 + 8u * (2 * nst + 5);
+  const int nslots = a.nsl << a.s.split;  // ring slots per tile
   constexpr uint32_t TMEM_COLS = 2 * NOUT < 32 ? 32 : 2 * NOUT;
 
   if (threadIdx.x == 0) {
@@ -1226,12 +1280,12 @@ __global__ void __launch_bounds__(TC_THREADS, 1) conv_gemm_tc_kernel(const GemmA
         if (!ok) break;
         tc_fence_after_sync();
         const uint32_t tmem_d = tmem_base + acc * NOUT;
-        for (int s = 0; s < a.nsl; ++s) {
+        for (int s = 0; s < nslots; ++s) {
           ok = mbar_wait(full_bar(st), ph, abort_flag, 0x12);
           if (!ok) break;
           tc_fence_after_sync();
           const uint64_t adesc = make_desc_sw128(stage0 + st * STAGE_BYTES, 16, 1024);
-          const uint64_t bdesc = make_desc_sw128(w0 + (uint32_t)(WRES ? s : st) * WSLICE, 16, 1024);
+          const uint64_t bdesc = make_desc_sw128(w0 + (uint32_t)(WRES ? s >> a.s.split : st) * WSLICE, 16, 1024);
 #pragma unroll
           for (int j = 0; j < 4; ++j)  // four K = 16 steps inside the 64-wide slice: +32 bytes each
             mma_bf16_ss(tmem_d, adesc + 2 * j, bdesc + 2 * j, idesc, (s | j) != 0);
@@ -1333,11 +1387,11 @@ __global__ void __launch_bounds__(TC_THREADS, 1) conv_gemm_tc_kernel(const GemmA
           bool ok = true;
           weights_ready();
           for (int tile = blockIdx.x; tile < a.t.tiles && ok; tile += gridDim.x) {
-            for (int s = 0; s < a.nsl; ++s) {
+            for (int s = 0; s < nslots; ++s) {
               ok = mbar_wait(empty_bar(st), ph ^ 1, abort_flag, 0x73);
               if (!ok) break;
               mbar_expect_tx(full_bar(st), WSLICE);
-              bulk_g2s(w0 + st * WSLICE, a.wimg + ((size_t)s * a.ncol + co0) * 8, WSLICE, full_bar(st));
+              bulk_g2s(w0 + st * WSLICE, a.wimg + ((size_t)(s >> a.s.split) * a.ncol + co0) * 8, WSLICE, full_bar(st));
               if (++st == (uint32_t)nst) { st = 0; ph ^= 1; }
             }
           }
@@ -1354,10 +1408,14 @@ __global__ void __launch_bounds__(TC_THREADS, 1) conv_gemm_tc_kernel(const GemmA
       producer_rowwise<false>(a.s, a.t, a.nsl, a.nsl, nst, stage0, full_bar(0), empty_bar(0),
                               (TapEnt*)(sm.extra + wbytes), abort_flag, warp - FIRST_PROD_WARP, lane,
                               0x36);
-    } else if (a.s.packed) {
-      producer_loop_packed<CSR, false>(a.s, a.t, a.nsl, a.nsl, nst, stage0, full_bar(0), empty_bar(0),
-                                  (TapEnt*)(sm.extra + wbytes), tabbar0, abort_flag,
-                                  warp - FIRST_PROD_WARP, lane, 0x35);
+    } else if (a.s.packed && (CSR || a.s.exact)) {
+      producer_loop_packed<CSR, false, true>(a.s, a.t, nslots, nslots, nst, stage0, full_bar(0), empty_bar(0),
+                                             (TapEnt*)(sm.extra + wbytes), tabbar0, abort_flag,
+                                             warp - FIRST_PROD_WARP, lane, 0x35);
+    } else if (!CSR && a.s.packed) {
+      producer_loop_packed<false, false, false>(a.s, a.t, a.nsl, a.nsl, nst, stage0, full_bar(0), empty_bar(0),
+                                                (TapEnt*)(sm.extra + wbytes), tabbar0, abort_flag,
+                                                warp - FIRST_PROD_WARP, lane, 0x38);
     } else if (a.s.interp == 0) {
       producer_loop_copy<CSR, false>(a.s, a.t, a.nsl, a.nsl, nst, stage0, full_bar(0), empty_bar(0),
                                      (TapEnt*)(sm.extra + wbytes), tabbar0, abort_flag,
@@ -1407,7 +1465,9 @@ __global__ void __launch_bounds__(TC_THREADS, 1) conv_wgrad_tc_kernel(const Gemm
   const uint32_t done_bar = bar0 + 8u * (2 * nst + 2 * GY_STAGES);
   const uint32_t tabbar0 = done_bar + 8u;
   // This CTA's share of the gradient: output channels [co0, co0 + NOUT) and the M = 128 tiles
-  // [j0, j0 + nmt) of the (tap, input channel) axis, i.e. slices [sl0, sl0 + nsl).
+  // [j0, j0 + nmt) of the (tap, input channel) axis, i.e. slices [sl0, sl0 + nsl).  With split rows a tile
+  // holds the two parts of ONE slice (a.nsl and all slice numbers here count ring slots, two to a slice):
+  // their products are added in the epilogue.
   const int co0 = blockIdx.z * NOUT;
   const int j0 = blockIdx.y * a.mtpg;
   const int nmt_all = (a.nsl + 1) / 2;
@@ -1568,7 +1628,10 @@ __global__ void __launch_bounds__(TC_THREADS, 1) conv_wgrad_tc_kernel(const Gemm
       const int q = warp & 3;
       const int m = q * 32 + lane;  // row of the M = 128 tile
       for (int j = 0; j < nmt; ++j) {
-        const int e = (sl0 + 2 * j) * 64 + m;  // element tap * C + ci of the gathered axis
+        // element tap * C + ci of the gathered axis
+        const int e = a.s.split ? (j0 + j) * 64 + (m & 63) : (sl0 + 2 * j) * 64 + m;
+        // (an infinite gradient times what rounding left of a value: the rounded value's product is the answer)
+        const bool rest = a.s.split && m >= 64;
         const bool live = e < a.s.KC;
         const int tap = live ? e / a.s.C : 0, ci = live ? e - tap * a.s.C : 0;
 #pragma unroll
@@ -1580,7 +1643,9 @@ __global__ void __launch_bounds__(TC_THREADS, 1) conv_wgrad_tc_kernel(const Gemm
 #pragma unroll
             for (int c = 0; c < 32; ++c) {
               const int co = co0 + cc * 32 + c;
-              if (co < a.ocol) atomicAdd(a.gw + ((long)co * a.s.C + ci) * a.s.K + tap, __uint_as_float(v[c]));
+              const float f = __uint_as_float(v[c]);
+              if (co < a.ocol && !(rest && !(fabsf(f) < INFINITY)))
+                atomicAdd(a.gw + ((long)co * a.s.C + ci) * a.s.K + tap, f);
             }
           }
         }
@@ -1604,10 +1669,14 @@ __global__ void __launch_bounds__(TC_THREADS, 1) conv_wgrad_tc_kernel(const Gemm
       producer_rowwise<true>(a.s, a.t, nsl, nsl_pad, nst, stage0, full_bar(0), empty_bar(0),
                              (TapEnt*)(sm.extra + (size_t)GY_STAGES * GYB), abort_flag,
                              warp - FIRST_PROD_WARP, lane, 0x64);
+    } else if (a.s.packed && a.s.exact) {
+      producer_loop_packed<false, true, true>(a.s, a.t, nsl, nsl_pad, nst, stage0, full_bar(0), empty_bar(0),
+                                              (TapEnt*)(sm.extra + (size_t)GY_STAGES * GYB), tabbar0, abort_flag,
+                                              warp - FIRST_PROD_WARP, lane, 0x63, sl0);
     } else if (a.s.packed) {
-      producer_loop_packed<false, true>(a.s, a.t, nsl, nsl_pad, nst, stage0, full_bar(0), empty_bar(0),
-                                 (TapEnt*)(sm.extra + (size_t)GY_STAGES * GYB), tabbar0,
-                                 abort_flag, warp - FIRST_PROD_WARP, lane, 0x63, sl0);
+      producer_loop_packed<false, true, false>(a.s, a.t, nsl, nsl_pad, nst, stage0, full_bar(0), empty_bar(0),
+                                               (TapEnt*)(sm.extra + (size_t)GY_STAGES * GYB), tabbar0, abort_flag,
+                                               warp - FIRST_PROD_WARP, lane, 0x66, sl0);
     } else if (a.s.interp == 0) {
       producer_loop_copy<false, true>(a.s, a.t, nsl, nsl_pad, nst, stage0, full_bar(0), empty_bar(0),
                                       (TapEnt*)(sm.extra + (size_t)GY_STAGES * GYB), tabbar0,
@@ -2057,6 +2126,16 @@ int tapmap_build_weighted_launch(const mc_desc* d, const void* map, const void* 
 
 // map != null: the kernel decodes the map itself; tab != null: prebuilt table (tapmap_build_launch)
 // The producer for nearest maps that lets the TMA unit fetch the rows: whole 64-channel blocks, a prebuilt table.
+//
+// Where float32 values have to reach the tensor cores in two parts: interpolated taps (and, in the input
+// gradient, every list sum) of layers with padded channel counts.  These layers ran on the CUDA cores before
+// they came here, with products and sums in float32; one part per value - what the layers with whole
+// 64-channel blocks have always had - would round each operand to 8 bits.  The weights, grad_output of the weight
+// gradient and nearest taps are bf16 as they are.
+static bool padded_channels(int c) { return c % 64 != 0; }
+static bool split_fwd(const mc_desc* d) { return padded_channels(d->C_out) && (d->interp == 1 || d->interp == 2); }
+static bool split_dgrad(const mc_desc* d) { return padded_channels(d->C_out) || padded_channels(d->C_in); }
+
 static bool gather_by_tma(const mc_desc* d, const void* x, const void* tab, CUtensorMap* tm) {
   return d->interp == 0 && d->C_in % 64 == 0 && tapmap_compact(d, tab) &&
          make_gather_map(tm, x, (long)d->B * d->IH * d->IW, d->C_in);
@@ -2080,7 +2159,9 @@ static int fwd_launch_impl(const mc_desc* d, const void* x, const void* map, con
   a.wimg = (const uint4*)ws; a.bias = (const bf16*)bias; a.y = (bf16*)y;
   a.nsl = fwd_slices(d);
   a.s.KC = d->K * d->C_in;
-  a.s.packed = d->C_in % 64 != 0;
+  a.s.split = split_fwd(d);
+  a.s.exact = padded_channels(d->C_out);
+  a.s.packed = d->C_in % 64 != 0 || a.s.split;
   a.ocol = d->C_out;
   a.ncol = pad64(d->C_out);
   a.relu = (d->flags & MC_FLAG_RELU) ? 1 : 0;
@@ -2102,7 +2183,7 @@ static int fwd_launch_impl(const mc_desc* d, const void* x, const void* map, con
     a.s.tab = (const TapEnt*)t;
   }
   a.full_cnt = N_PRODUCER_WARPS;
-  if (a.s.tab && rowwise_shape(d) && p.nst >= ROW_TEAMS) {
+  if (a.s.tab && rowwise_shape(d) && p.nst >= ROW_TEAMS && !a.s.split) {
     a.s.packed = 2;
     a.full_cnt = N_PRODUCER_WARPS / ROW_TEAMS;
     a.s.tab32 = tapmap_compact(d, a.s.tab);
@@ -2235,7 +2316,8 @@ int conv_tc_dgrad_launch(const mc_desc* d, const void* gy, const void* inv, cons
   a.wimg = (const uint4*)ws; a.bias = (const bf16*)bias_out; a.y = (bf16*)gx;
   a.nsl = dgrad_slices(d);
   a.s.KC = d->K * d->C_out;
-  a.s.packed = d->C_out % 64 != 0;
+  a.s.split = a.s.exact = split_dgrad(d);
+  a.s.packed = a.s.split;
   a.ocol = d->C_in;
   a.ncol = pad64(d->C_in);
   a.relu = (bias_out && (d->flags & MC_FLAG_RELU)) ? 1 : 0;  // the transposed layer's forward
@@ -2261,7 +2343,7 @@ struct WgradPlan {
 
 static bool plan_wgrad(const mc_desc* d, size_t tabb, WgradPlan& p) {
   if (d->C_out % 8 != 0 || (long)d->K * d->C_in >= (1L << 24)) return false;
-  const int nsl = fwd_slices(d);
+  const int nsl = fwd_slices(d) << split_fwd(d);  // (ring slots)
   const int nmt = (nsl + 1) / 2;
   p.nout = pad64(d->C_out) % 128 == 0 ? 128 : 64;
   p.chunks = pad64(d->C_out) / p.nout;
@@ -2319,9 +2401,11 @@ static int wgrad_launch_impl(const mc_desc* d, const void* gy, const void* x, co
   a.s.tab = (const TapEnt*)tab;
   if (!make_tiling(a.t, d->B, d->OH, d->OW)) return MC_ERR_TOO_LARGE;
   a.gy = (const bf16*)gy; a.gw = (float*)gw; a.gb = (float*)gb;
-  a.nsl = fwd_slices(d);
+  a.s.split = split_fwd(d);
+  a.s.exact = padded_channels(d->C_out);
+  a.nsl = fwd_slices(d) << a.s.split;
   a.s.KC = d->K * d->C_in;
-  a.s.packed = d->C_in % 64 != 0;
+  a.s.packed = d->C_in % 64 != 0 || a.s.split;
   a.ocol = d->C_out;
   a.ncol = pad64(d->C_out);
   WgradPlan p;
@@ -2332,7 +2416,7 @@ static int wgrad_launch_impl(const mc_desc* d, const void* gy, const void* x, co
   a.nst = p.nst;
   a.mtpg = p.mtpg;
   a.full_cnt = N_PRODUCER_WARPS;
-  if (tab && rowwise_shape(d) && p.nst >= ROW_TEAMS) {
+  if (tab && rowwise_shape(d) && p.nst >= ROW_TEAMS && !a.s.split) {
     a.s.packed = 2;
     a.full_cnt = N_PRODUCER_WARPS / ROW_TEAMS;
     a.s.tab32 = tapmap_compact(d, tab);

@@ -14,10 +14,7 @@ def _case(cin, cout, interp, seed):
     B, IH, IW, OH, OW, K = 2, 10, 13, 9, 17, 5
     bf = lambda *s: torch.randn(*s, generator=g).to(torch.bfloat16)
     m = (torch.rand(OH, OW, K, 2, generator=g) * torch.tensor([IW + 1.0, IH + 1.0]) - 1.0).contiguous()
-    # tap 1 reads the same place from six grid pixels in a row: inverse lists beyond a table record's four
-    # entries.  (Not from all of them: the gathered sum is rounded to bf16, so that a list of n entries of
-    # N(0, 1) adds an error of 2^-9 sqrt(n) |w| sqrt(C_out) to an output of about sqrt(K C_out) |w| - 1e-3
-    # of it for six, and beyond the tolerance at its tails for all 153.)
+    # tap 1 reads the same place from six grid pixels in a row: inverse lists beyond a table record's four entries
     flat = m.view(OH * OW, K, 2)
     flat[:, 1] = flat[(torch.arange(OH * OW) // 6) * 6, 1]
     w = (torch.randn(cout, cin, K, generator=g) / (cin * K) ** 0.5).to(torch.bfloat16)
@@ -41,6 +38,59 @@ def test_odd_channel_counts_against_oracle(cin, cout, interp, layout):
     for name, a, r in (("y", y, want), ("gx", g[0], want_g[0]), ("gw", g[1], want_g[1]), ("gb", g[2], want_g[2])):
         H.assert_close(a.float(), r, H.TOL[torch.bfloat16], name)
     assert host.impl.device_status() == 0
+
+
+def _run(x, gy, w, b, m, K, interp, iw=None):
+    from mappedconvolutions_b200 import host
+    cl = lambda t: t.cuda().contiguous(memory_format=torch.channels_last)
+    maps, pre = ((m.cuda(),), "mapped_conv") if iw is None else ((m.cuda(), iw.cuda()), "weighted_mapped_conv")
+    y = getattr(host.impl, pre + "_forward")(cl(x), *maps, w.cuda(), b.cuda(), K, interp)
+    g = getattr(host.impl, pre + "_backward")(cl(gy), *maps, cl(x), w.cuda(), b.cuda(), K, interp)
+    assert host.impl.device_status() == 0
+    return [t.float().cpu() for t in (y, g[0], g[1])]
+
+
+def _oracle(x, gy, w, b, m, K, interp, iw=None):
+    maps, pre = ((m,), "mapped_conv") if iw is None else ((m, iw), "weighted_mapped_conv")
+    y = getattr(oracle, pre + "_forward")(x, *maps, w, b, K, interp)
+    return [y] + list(getattr(oracle, pre + "_backward")(gy, *maps, x, w, b, K, interp)[:2])
+
+
+# Padded channel counts keep float32 products and sums up to the one rounding of the result.  Bound: that rounding
+# (2^-8 of the value), plus 2^-15 of the sum of the terms' magnitudes: 2^-16 for values that reach the tensor
+# cores as two bf16 parts, and as much for float32 sums of up to 1600 terms, whose errors mostly cancel.
+@pytest.mark.parametrize("interp,P", [(0, 0), (1, 0), (2, 0), (0, 3)])
+@pytest.mark.parametrize("cin,cout", [(32, 32), (96, 64), (64, 96), (32, 64), (128, 200), (3, 40), (12, 72), (8, 8)])
+def test_odd_channel_counts_round_once(cin, cout, interp, P):
+    x, gy, w, b, m, K, _ = _case(cin, cout, interp, cin + cout)
+    g = torch.Generator().manual_seed(1)
+    # tap 2 reads one place from every grid pixel: lists of 153 entries
+    m.view(-1, K, 2)[:, 2] = torch.tensor([4.25, 3.5])
+    iw = None
+    if P:
+        m = (m.unsqueeze(3) + torch.rand(*m.shape[:3], P, 2, generator=g) * 3).contiguous()
+        iw = torch.rand(*m.shape[:3], P, generator=g)
+    d = lambda *ts: [None if t is None else t.double() for t in ts]
+    got = _run(x, gy, w, b, m, K, interp, iw)
+    xd, gd, wd, bd, md, iwd = d(x, gy, w, b, m, iw)
+    want = _oracle(xd, gd, wd, bd, md, K, interp, iwd)
+    size = _oracle(xd.abs(), gd.abs(), wd.abs(), bd.abs(), md, K, interp, iwd)
+    for name, a, r, s in zip(("y", "gx", "gw"), got, want, size):
+        if name != "gx" and cout % 64 == 0 and (interp or P):
+            continue  # (only the image's channels are padded: interpolated taps are bf16 there, as in whole blocks)
+        over = ((a.double() - r).abs() / (2.0 ** -8 * r.abs() + 2.0 ** -15 * s + 1e-30)).max().item()
+        assert over <= 1.0, (name, over)
+
+
+@pytest.mark.parametrize("interp", [0, 1])
+@pytest.mark.parametrize("cin,cout", [(32, 32), (64, 96), (8, 40), (3, 24)])
+def test_infinities_reach_what_uses_them(cin, cout, interp):
+    x, gy, w, b, m, K, _ = _case(cin, cout, interp, cin)
+    x[0, 0, 0, 0], x[1, 1, 5, 7], gy[0, 0, 0, 0], gy[1, 2, 4, 4] = float("inf"), float("nan"), float("inf"), -float("inf")
+    f = [t.float() for t in (x, gy, w, b)]
+    for name, a, r in zip(("y", "gx", "gw"), _run(x, gy, w, b, m, K, interp), _oracle(*f, m, K, interp)):
+        assert torch.equal(a.isnan(), r.isnan()) and torch.equal(a.isinf(), r.isinf()), name
+        assert torch.equal(a[a.isinf()], r[r.isinf()]), name
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
