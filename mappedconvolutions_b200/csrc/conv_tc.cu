@@ -157,6 +157,12 @@ struct GemmArgs {
   int relu;           // fwd: y = max(0, .) after the bias
 };
 
+// max(0, v) that keeps NaN, as torch's activation does
+__device__ __forceinline__ float relu_nan(float v) {
+  asm("max.NaN.f32 %0, %0, 0f00000000;" : "+f"(v));
+  return v;
+}
+
 __device__ __forceinline__ void blend4(const uint4& v, float w, float (&acc)[8]) {
   bf16x2_fma(v.x, w, acc[0], acc[1]);
   bf16x2_fma(v.y, w, acc[2], acc[3]);
@@ -1355,7 +1361,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) conv_gemm_tc_kernel(const GemmA
 #pragma unroll
           for (int e = 0; e < 8; ++e) {
             f[e] = __uint_as_float(v[j * 8 + e]) + bs[e];
-            if (a.relu) f[e] = fmaxf(f[e], 0.f);
+            if (a.relu) f[e] = relu_nan(f[e]);
           }
           o.x = pack_bf16x2(f[0], f[1]);
           o.y = pack_bf16x2(f[2], f[3]);

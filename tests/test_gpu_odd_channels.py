@@ -93,6 +93,23 @@ def test_infinities_reach_what_uses_them(cin, cout, interp):
         assert torch.equal(a[a.isinf()], r[r.isinf()]), name
 
 
+@pytest.mark.parametrize("weighted", [False, True])
+@pytest.mark.parametrize("cout", [64, 40])
+def test_fused_activation_keeps_nan(cout, weighted):
+    from mappedconvolutions_b200 import nn as mnn
+    x, _, w, b, m, K, _ = _case(64, cout, 0, 3)
+    x[0, 5, 4, 4] = float("nan")
+    args = (m.cuda(),)
+    if weighted:
+        args = (m.unsqueeze(3).repeat(1, 1, 1, 3, 1).cuda(), torch.rand(*m.shape[:3], 3).cuda())
+    layers = [mnn.MappedConvolution(64, cout, K, "nearest", activation=a).cuda().bfloat16() for a in (None, "relu")]
+    layers[1].load_state_dict(layers[0].state_dict())
+    xc = x.cuda().contiguous(memory_format=torch.channels_last)
+    want, got = torch.relu(layers[0](xc, *args)), layers[1](xc, *args)
+    assert want.isnan().any() and torch.equal(want.isnan(), got.isnan())
+    assert torch.equal(want.nan_to_num(), got.nan_to_num())
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("B,C,H_,W_", [(1, 64, 8, 8), (3, 65, 7, 9), (2, 17, 1, 130), (2, 3, 5, 7), (1, 200, 3, 3), (5, 16, 1, 1),
                                        (1, 20, 64, 65)])
