@@ -902,10 +902,11 @@ bool seen_by_torch(std::initializer_list<const Tensor*> ts) {
   return false;
 }
 
+// (a map or point weights that require a gradient make the output require one too; their own stays undefined)
 bool records(std::initializer_list<const Tensor*> ts) {
   if (!at::GradMode::is_enabled()) return false;
   for (const Tensor* t : ts)
-    if (t->defined() && t->requires_grad()) return true;
+    if (t && t->defined() && t->requires_grad()) return true;
   return false;
 }
 OptTensor as_opt(const Tensor& t) { return t.defined() ? OptTensor(t) : OptTensor(); }
@@ -968,7 +969,7 @@ struct MaxPoolFn : torch::autograd::Function<MaxPoolFn> {
   }
   static variable_list backward(AutogradContext* ctx, variable_list g) {
     variable_list out(5);
-    if (!g[0].defined()) return out;
+    if (!g[0].defined() || !ctx->needs_input_grad(0)) return out;
     const auto s = ctx->get_saved_variables();
     out[0] = max_unpool(g[0], s[0], s[1], as_opt(s[2]), ctx->saved_data["h"].toInt(), ctx->saved_data["w"].toInt(),
                         ctx->saved_data["k"].toInt(), ctx->saved_data["i"].toInt());
@@ -999,8 +1000,9 @@ struct LinearFn : torch::autograd::Function<LinearFn> {
     return run_linear(op, x, map, iw, oh, ow, K, interp);
   }
   static variable_list backward(AutogradContext* ctx, variable_list g) {
-    const auto s = ctx->get_saved_variables();
     variable_list out(8);
+    if (!ctx->needs_input_grad(0)) return out;
+    const auto s = ctx->get_saved_variables();
     // (upstream gradients come in any layout; the ops want one of the two)
     const Tensor gy = g[0].is_contiguous() || g[0].is_contiguous(at::MemoryFormat::ChannelsLast) ? g[0] : g[0].contiguous();
     out[0] = run_linear(ctx->saved_data["o"].toInt(), gy, s[0], as_opt(s[1]), ctx->saved_data["h"].toInt(),
@@ -1011,7 +1013,7 @@ struct LinearFn : torch::autograd::Function<LinearFn> {
 OptTensor linear_layer(int64_t op, const Tensor& x, const Tensor& map, const OptTensor& iw, int64_t oh, int64_t ow,
                        int64_t K, int64_t interp) {
   if (seen_by_torch({&x, &map, opt(iw)})) return c10::nullopt;
-  if (!records({&x})) return run_linear(op, x, map, iw, oh, ow, K, interp);
+  if (!records({&x, &map, opt(iw)})) return run_linear(op, x, map, iw, oh, ow, K, interp);
   return LinearFn::apply(x, map, iw, op, oh, ow, K, interp);
 }
 
@@ -1120,19 +1122,19 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("conv_layer", [](const Tensor& x, const Tensor& w, const Tensor& b, const Tensor& map, int64_t k, int64_t i,
                          const OptTensor& iw, bool relu) -> OptTensor {
     if (seen_by_torch({&x, &w, &b, &map, opt(iw)})) return c10::nullopt;
-    if (!records({&x, &w, &b})) return conv_forward(x, map, iw, w, b, k, i, false, relu);
+    if (!records({&x, &w, &b, &map, opt(iw)})) return conv_forward(x, map, iw, w, b, k, i, false, relu);
     return ConvFn::apply(x, w, b, map, iw, k, i, relu);
   });
   m.def("tconv_layer", [](const Tensor& x, const Tensor& w, const Tensor& b, const Tensor& map, int64_t oh, int64_t ow,
                           int64_t k, int64_t i, const OptTensor& iw) -> OptTensor {
     if (seen_by_torch({&x, &w, &b, &map, opt(iw)})) return c10::nullopt;
-    if (!records({&x, &w, &b})) return tconv_forward(x, map, iw, w, b, oh, ow, k, i);
+    if (!records({&x, &w, &b, &map, opt(iw)})) return tconv_forward(x, map, iw, w, b, oh, ow, k, i);
     return TconvFn::apply(x, w, b, map, iw, oh, ow, k, i);
   });
   m.def("max_pool_layer", [](const Tensor& x, const Tensor& map, int64_t k, int64_t i,
                              const OptTensor& iw) -> c10::optional<std::tuple<Tensor, Tensor>> {
     if (seen_by_torch({&x, &map, opt(iw)})) return c10::nullopt;
-    auto r = records({&x}) ? MaxPoolFn::apply(x, map, iw, k, i) : max_pool(x, map, iw, k, i);
+    auto r = records({&x, &map, opt(iw)}) ? MaxPoolFn::apply(x, map, iw, k, i) : max_pool(x, map, iw, k, i);
     return std::make_tuple(r[0], r[1]);
   });
   m.def("avg_pool_layer", [](const Tensor& x, const Tensor& map, int64_t k, int64_t i, const OptTensor& iw) {
