@@ -1022,13 +1022,20 @@ OptTensor linear_layer(int64_t op, const Tensor& x, const Tensor& map, const Opt
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   namespace py = pybind11;
   m.doc() = "mapped convolution ops on the sm_100a C-ABI library (reference pybind surface)";
+  // Calls run without the interpreter lock, as the backward nodes do: plans are built under plan_mutex, and the
+  // allocator, a dispatch mode or a tracing hook may want the lock there - a caller that kept it while it waits
+  // for plan_mutex would never give it back.
+  auto def = [&m](const char* name, auto&& f, auto&&... extra) {
+    m.def(name, std::forward<decltype(f)>(f), std::forward<decltype(extra)>(extra)...,
+          py::call_guard<py::gil_scoped_release>());
+  };
   // MappedConvForward / Backward, include/nn/layers/mapped_convolution_layer.h:64-88, :90-135
-  m.def("mapped_conv_forward",
+  def("mapped_conv_forward",
         [](const Tensor& x, const Tensor& map, const Tensor& w, const Tensor& b, int64_t k, int64_t i,
            bool relu) { return conv_forward(x, map, c10::nullopt, w, b, k, i, false, relu); },
         py::arg("input"), py::arg("sample_map"), py::arg("weight"), py::arg("bias"),
         py::arg("kernel_size"), py::arg("interpolation"), py::arg("relu") = false);
-  m.def("mapped_conv_backward",
+  def("mapped_conv_backward",
         [](const Tensor& gy, const Tensor& map, const Tensor& x, const Tensor& w, const Tensor& b,
            int64_t k, int64_t i, bool need_input_grad, bool need_weight_grad,
            const c10::optional<Tensor>& relu_output) {
@@ -1040,124 +1047,124 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         py::arg("need_input_grad") = true, py::arg("need_weight_grad") = true,
         py::arg("relu_output") = py::none());
   // include/nn/layers/weighted_mapped_convolution_layer.h:65-93, :95-150
-  m.def("weighted_mapped_conv_forward",
+  def("weighted_mapped_conv_forward",
         [](const Tensor& x, const Tensor& map, const Tensor& iw, const Tensor& w, const Tensor& b,
            int64_t k, int64_t i) { return conv_forward(x, map, iw, w, b, k, i); });
-  m.def("weighted_mapped_conv_backward",
+  def("weighted_mapped_conv_backward",
         [](const Tensor& gy, const Tensor& map, const Tensor& iw, const Tensor& x, const Tensor& w,
            const Tensor& b, int64_t k, int64_t i) {
           return conv_backward(gy, map, iw, x, w, b, k, i, true);
         });
   // include/nn/layers/mapped_transposed_convolution_layer.h:64-92, :94-143
-  m.def("mapped_transposed_conv_forward",
+  def("mapped_transposed_conv_forward",
         [](const Tensor& x, const Tensor& map, const Tensor& w, const Tensor& b, int64_t oh,
            int64_t ow, int64_t k, int64_t i) {
           return tconv_forward(x, map, c10::nullopt, w, b, oh, ow, k, i);
         });
-  m.def("mapped_transposed_conv_backward",
+  def("mapped_transposed_conv_backward",
         [](const Tensor& gy, const Tensor& map, const Tensor& x, const Tensor& w, const Tensor& b,
            int64_t k, int64_t i) { return tconv_backward(gy, map, c10::nullopt, x, w, b, k, i); });
   // include/nn/layers/weighted_mapped_transposed_convolution_layer.h:66-98, :100-155
-  m.def("weighted_mapped_transposed_conv_forward",
+  def("weighted_mapped_transposed_conv_forward",
         [](const Tensor& x, const Tensor& map, const Tensor& iw, const Tensor& w, const Tensor& b,
            int64_t oh, int64_t ow, int64_t k, int64_t i) {
           return tconv_forward(x, map, iw, w, b, oh, ow, k, i);
         });
-  m.def("weighted_mapped_transposed_conv_backward",
+  def("weighted_mapped_transposed_conv_backward",
         [](const Tensor& gy, const Tensor& map, const Tensor& iw, const Tensor& x, const Tensor& w,
            const Tensor& b, int64_t k, int64_t i) { return tconv_backward(gy, map, iw, x, w, b, k, i); });
   // include/nn/layers/mapped_max_pooling_layer.h:46-71, :73-98 and the weighted variants
-  m.def("mapped_max_pool", [](const Tensor& x, const Tensor& map, int64_t k, int64_t i) {
+  def("mapped_max_pool", [](const Tensor& x, const Tensor& map, int64_t k, int64_t i) {
     return max_pool(x, map, c10::nullopt, k, i);
   });
-  m.def("mapped_max_unpool", [](const Tensor& gy, const Tensor& idx, const Tensor& map, int64_t ih,
+  def("mapped_max_unpool", [](const Tensor& gy, const Tensor& idx, const Tensor& map, int64_t ih,
                                 int64_t iw_, int64_t k, int64_t i) {
     return max_unpool(gy, idx, map, c10::nullopt, ih, iw_, k, i);
   });
-  m.def("weighted_mapped_max_pool",
+  def("weighted_mapped_max_pool",
         [](const Tensor& x, const Tensor& map, const Tensor& iw, int64_t k, int64_t i) {
           return max_pool(x, map, iw, k, i);
         });
-  m.def("weighted_mapped_max_unpool",
+  def("weighted_mapped_max_unpool",
         [](const Tensor& gy, const Tensor& idx, const Tensor& map, const Tensor& iw, int64_t ih,
            int64_t iw_, int64_t k, int64_t i) { return max_unpool(gy, idx, map, iw, ih, iw_, k, i); });
   // include/nn/layers/mapped_avg_pooling_layer.h:42-64, :66-88 and the weighted variants
-  m.def("mapped_avg_pool", [](const Tensor& x, const Tensor& map, int64_t k, int64_t i) {
+  def("mapped_avg_pool", [](const Tensor& x, const Tensor& map, int64_t k, int64_t i) {
     return avg_pool(x, map, c10::nullopt, k, i);
   });
-  m.def("mapped_avg_unpool", [](const Tensor& gy, const Tensor& map, int64_t ih, int64_t iw_,
+  def("mapped_avg_unpool", [](const Tensor& gy, const Tensor& map, int64_t ih, int64_t iw_,
                                 int64_t k, int64_t i) {
     return avg_unpool(gy, map, c10::nullopt, ih, iw_, k, i);
   });
-  m.def("weighted_mapped_avg_pool",
+  def("weighted_mapped_avg_pool",
         [](const Tensor& x, const Tensor& map, const Tensor& iw, int64_t k, int64_t i) {
           return avg_pool(x, map, iw, k, i);
         });
-  m.def("weighted_mapped_avg_unpool",
+  def("weighted_mapped_avg_unpool",
         [](const Tensor& gy, const Tensor& map, const Tensor& iw, int64_t ih, int64_t iw_, int64_t k,
            int64_t i) { return avg_unpool(gy, map, iw, ih, iw_, k, i); });
   // ResampleToMap (scatter) / ResampleFromMap (gather), include/nn/layers/resample_layer.h:38-80,
   // and include/nn/layers/weighted_resample_layer.h:49-103
-  m.def("resample_to_map", [](const Tensor& x, const Tensor& map, int64_t oh, int64_t ow, int64_t i) {
+  def("resample_to_map", [](const Tensor& x, const Tensor& map, int64_t oh, int64_t ow, int64_t i) {
     return resample_to(x, map, c10::nullopt, oh, ow, i);
   });
-  m.def("resample_from_map", [](const Tensor& x, const Tensor& map, int64_t i) {
+  def("resample_from_map", [](const Tensor& x, const Tensor& map, int64_t i) {
     return resample_from(x, map, c10::nullopt, i);
   });
-  m.def("weighted_resample_to_map", [](const Tensor& x, const Tensor& map, const Tensor& iw,
+  def("weighted_resample_to_map", [](const Tensor& x, const Tensor& map, const Tensor& iw,
                                        int64_t oh, int64_t ow, int64_t i) {
     return resample_to(x, map, iw, oh, ow, i);
   });
-  m.def("weighted_resample_from_map",
+  def("weighted_resample_from_map",
         [](const Tensor& x, const Tensor& map, const Tensor& iw, int64_t i) {
           return resample_from(x, map, iw, i);
         });
   // KNNForward, include/util/layers/knn_layer.h:25-35 -> [idx (B,k,N) int64 1-based, dist]
-  m.def("knn_forward", &knn_forward);
+  def("knn_forward", &knn_forward);
   // Cube2RectForward, include/util/layers/cube2rect_layer.h:14-45
-  m.def("cube2rect", &cube2rect);
+  def("cube2rect", &cube2rect);
   // VotingResampleToMap, include/nn/layers/voting_resample_layer.h:34-58
-  m.def("voting_resample_to_map", &voting_resample_to_map);
+  def("voting_resample_to_map", &voting_resample_to_map);
   // differentiable calls of the layer API (None: see seen_by_torch)
-  m.def("conv_layer", [](const Tensor& x, const Tensor& w, const Tensor& b, const Tensor& map, int64_t k, int64_t i,
+  def("conv_layer", [](const Tensor& x, const Tensor& w, const Tensor& b, const Tensor& map, int64_t k, int64_t i,
                          const OptTensor& iw, bool relu) -> OptTensor {
     if (seen_by_torch({&x, &w, &b, &map, opt(iw)})) return c10::nullopt;
     if (!records({&x, &w, &b, &map, opt(iw)})) return conv_forward(x, map, iw, w, b, k, i, false, relu);
     return ConvFn::apply(x, w, b, map, iw, k, i, relu);
   });
-  m.def("tconv_layer", [](const Tensor& x, const Tensor& w, const Tensor& b, const Tensor& map, int64_t oh, int64_t ow,
+  def("tconv_layer", [](const Tensor& x, const Tensor& w, const Tensor& b, const Tensor& map, int64_t oh, int64_t ow,
                           int64_t k, int64_t i, const OptTensor& iw) -> OptTensor {
     if (seen_by_torch({&x, &w, &b, &map, opt(iw)})) return c10::nullopt;
     if (!records({&x, &w, &b, &map, opt(iw)})) return tconv_forward(x, map, iw, w, b, oh, ow, k, i);
     return TconvFn::apply(x, w, b, map, iw, oh, ow, k, i);
   });
-  m.def("max_pool_layer", [](const Tensor& x, const Tensor& map, int64_t k, int64_t i,
+  def("max_pool_layer", [](const Tensor& x, const Tensor& map, int64_t k, int64_t i,
                              const OptTensor& iw) -> c10::optional<std::tuple<Tensor, Tensor>> {
     if (seen_by_torch({&x, &map, opt(iw)})) return c10::nullopt;
     auto r = records({&x, &map, opt(iw)}) ? MaxPoolFn::apply(x, map, iw, k, i) : max_pool(x, map, iw, k, i);
     return std::make_tuple(r[0], r[1]);
   });
-  m.def("avg_pool_layer", [](const Tensor& x, const Tensor& map, int64_t k, int64_t i, const OptTensor& iw) {
+  def("avg_pool_layer", [](const Tensor& x, const Tensor& map, int64_t k, int64_t i, const OptTensor& iw) {
     return linear_layer(0, x, map, iw, 0, 0, k, i);
   });
-  m.def("avg_unpool_layer", [](const Tensor& x, int64_t oh, int64_t ow, const Tensor& map, int64_t k, int64_t i,
+  def("avg_unpool_layer", [](const Tensor& x, int64_t oh, int64_t ow, const Tensor& map, int64_t k, int64_t i,
                                const OptTensor& iw) { return linear_layer(1, x, map, iw, oh, ow, k, i); });
-  m.def("resample_layer", [](const Tensor& x, const Tensor& map, std::pair<int64_t, int64_t> shape, int64_t i,
+  def("resample_layer", [](const Tensor& x, const Tensor& map, std::pair<int64_t, int64_t> shape, int64_t i,
                              const OptTensor& iw) {
     return linear_layer(2, x, map, iw, shape.first, shape.second, 1, i);
   });
-  m.def("unresample_layer", [](const Tensor& x, const Tensor& map, int64_t i, const OptTensor& iw) {
+  def("unresample_layer", [](const Tensor& x, const Tensor& map, int64_t i, const OptTensor& iw) {
     return linear_layer(3, x, map, iw, 0, 0, 1, i);
   });
-  m.def("clear_plan_cache", &clear_plan_cache);
-  m.def("plan_cache_kinds", &plan_cache_kinds);
+  def("clear_plan_cache", &clear_plan_cache);
+  def("plan_cache_kinds", &plan_cache_kinds);
   // Row plans (the fast path for maps that are translation invariant along image rows) on / off;
   // returns the previous setting.  Off: every map takes the general kernels.
-  m.def("set_row_plans", [](bool on) { const bool was = g_row_plans; g_row_plans = on; return was; });
+  def("set_row_plans", [](bool on) { const bool was = g_row_plans; g_row_plans = on; return was; });
   // Synchronises the current stream and returns the device status word (0 = every kernel ran to
   // completion; otherwise the code of the first bounded device-side wait that ran out, after which
   // the kernel returned early and its output is invalid).  reset clears the word.
-  m.def("device_status", [](bool reset) { return mc_device_status(cur_stream(), reset ? 1 : 0); },
+  def("device_status", [](bool reset) { return mc_device_status(cur_stream(), reset ? 1 : 0); },
         py::arg("reset") = true);
-  m.def("abi_version", []() { return mc_abi_version(); });
+  def("abi_version", []() { return mc_abi_version(); });
 }
