@@ -21,8 +21,15 @@
  *  - alignment: the bf16 tensor-core paths (MC_BF16 + MC_NHWC, C_out % 64 == 0, every *_tap, *_inv and
  *    *_rowplan entry point, mc_conv_fwd_static_scratch) move 16 bytes at a time and return
  *    MC_ERR_BAD_ARG for a tensor, map, table or workspace pointer that is not 16-byte aligned; the
- *    generic kernels take any element-aligned pointer;
- *  - finite inputs: the bf16 tensor-core kernels gather without predicates - a corner or tap that
+ *    generic kernels take any element-aligned pointer.  mc_conv_fwd / mc_conv_wgrad and their transposed forms use
+ *    the tensor cores for other multiples of 8 output channels too where alignment and workspace allow, and the
+ *    generic kernels where they do not;
+ *  - precision of MC_BF16: sums are float32, results are rounded once.  On the tensor cores an interpolated value,
+ *    and a sum of grad_output values in the input gradient, is rounded to bf16 before it is multiplied where the
+ *    channel counts are multiples of 64 (C_out for forward and weight gradient, both for the input gradient);
+ *    with other counts it keeps 16 significant bits;
+ *  - finite inputs: the bf16 tensor-core kernels for channel counts that are multiples of 64 gather without
+ *    predicates - a corner or tap that
  *    contributes nothing still reads a real pixel (pixel 0 of the image for a tap that lies outside
  *    it completely) and multiplies it by zero.  The reference skips such corners
  *    (include/core/interpolation.h:125-154); results agree for finite inputs, a NaN or infinity
@@ -187,7 +194,7 @@ int mc_tapmap_build_weighted(const mc_desc* d, const void* map, const void* iw, 
 int mc_invmap_build_weighted(const mc_desc* d, const void* map, const void* iw, void* inv, size_t inv_bytes,
                              void* ws, size_t ws_bytes, void* stream);
 /* Same result as mc_conv_dgrad, computed on the tensor cores from a prebuilt inverse map.
- * bf16, MC_NHWC, C_in % 64 == 0, C_out % 64 == 0 (mc_conv_dgrad_inv_supported() tells).
+ * bf16, MC_NHWC, C_in % 8 == 0, C_out % 8 == 0 (mc_conv_dgrad_inv_supported() tells).
  * Replaces cuda::MappedConvBackwardInput, src/nn/cuda/mapped_convolution_layer.cu:75-132. */
 int mc_conv_dgrad_inv_supported(const mc_desc* d);
 size_t mc_conv_dgrad_inv_workspace_bytes(const mc_desc* d);

@@ -87,6 +87,12 @@ int mc_device_status(void* stream, int reset) {
   return device_status_read((cudaStream_t)stream, reset);
 }
 
+// Layers with padded output channels ask for a workspace and for aligned tensors only to be faster: without
+// them the generic kernels do the work.  (These codes come from checks, before anything is launched.)
+static bool generic_takes(const mc_desc* d, int rc) {
+  return d->C_out % 64 != 0 && (rc == MC_ERR_WORKSPACE || rc == MC_ERR_BAD_ARG || rc == MC_ERR_TOO_LARGE);
+}
+
 size_t mc_conv_fwd_workspace_bytes(const mc_desc* d) {
   if (!d || check_conv_desc_public(d)) return 0;
   return conv_tc_fwd_supported(d) ? conv_tc_fwd_ws(d) : 0;
@@ -98,7 +104,10 @@ int mc_conv_fwd(const mc_desc* d, const void* x, const void* map, const void* iw
   if (rc) return rc;
   if (!x || !map || !w || !y || (d->P > 0 && !iw)) return MC_ERR_BAD_ARG;
   cudaStream_t st = (cudaStream_t)stream;
-  if (conv_tc_fwd_supported(d)) return conv_tc_fwd_launch(d, x, map, w, bias, y, ws, ws_bytes, st);
+  if (conv_tc_fwd_supported(d)) {
+    rc = conv_tc_fwd_launch(d, x, map, w, bias, y, ws, ws_bytes, st);
+    if (!generic_takes(d, rc)) return rc;
+  }
   return conv_fwd_simt_launch(d, x, map, iw, w, bias, y, st);
 }
 
@@ -311,7 +320,10 @@ int mc_conv_wgrad(const mc_desc* d, const void* gy, const void* x, const void* m
   if (rc) return rc;
   if (!gy || !x || !map || !gw || (d->P > 0 && !iw)) return MC_ERR_BAD_ARG;
   cudaStream_t st = (cudaStream_t)stream;
-  if (conv_tc_wgrad_supported(d)) return conv_tc_wgrad_launch(d, gy, x, map, gw, gb, ws, ws_bytes, st);
+  if (conv_tc_wgrad_supported(d)) {
+    rc = conv_tc_wgrad_launch(d, gy, x, map, gw, gb, ws, ws_bytes, st);
+    if (!generic_takes(d, rc)) return rc;
+  }
   rc = conv_wgrad_simt_launch(d, gy, x, map, iw, gw, st);
   if (rc) return rc;
   if (gb) rc = bias_grad_launch(d, gy, gb, st);

@@ -1995,8 +1995,23 @@ static int fwd_slices(const mc_desc* d) { return (int)(((long)d->K * d->C_in + 6
 // (128 -> 96 channels on 3 x 433 x 866 pixels: 50.7 ms).
 static int pad64(int c) { return (c + 63) & ~63; }
 
+// Where float32 values have to reach the tensor cores in two parts: interpolated taps (and, in the input
+// gradient, every list sum) of layers with padded channel counts.  These layers ran on the CUDA cores before
+// they came here, with products and sums in float32; one part per value - what the layers with whole
+// 64-channel blocks have always had - would round each operand to 8 bits.  The weights, grad_output of the weight
+// gradient and nearest taps are bf16 as they are.
+static bool padded_channels(int c) { return c % 64 != 0; }
+static bool split_fwd(const mc_desc* d) { return padded_channels(d->C_out) && (d->interp == 1 || d->interp == 2); }
+static bool split_dgrad(const mc_desc* d) { return padded_channels(d->C_out) || padded_channels(d->C_in); }
+
+// Pixel indices of a batch in 30 bits; larger batches of padded layers stay with the CUDA cores.
+static bool indexable(const mc_desc* d) {
+  return (long)d->B * d->IH * d->IW < (1L << 30) && (long)d->B * d->OH * d->OW < (1L << 30);
+}
+
 bool conv_tc_fwd_supported(const mc_desc* d) {
   if (d->dtype != MC_BF16 || d->layout != MC_NHWC || d->P != 0) return false;
+  if (padded_channels(d->C_out) && !indexable(d)) return false;
   if (d->C_out % 8 != 0 || (long)d->K * d->C_in >= (1L << 24)) return false;
   GemmPlan p;
   return plan_gemm(pad64(d->C_out), fwd_slices(d), d->K, p);
@@ -2130,23 +2145,13 @@ int tapmap_build_weighted_launch(const mc_desc* d, const void* map, const void* 
   return MC_OK;
 }
 
-// map != null: the kernel decodes the map itself; tab != null: prebuilt table (tapmap_build_launch)
 // The producer for nearest maps that lets the TMA unit fetch the rows: whole 64-channel blocks, a prebuilt table.
-//
-// Where float32 values have to reach the tensor cores in two parts: interpolated taps (and, in the input
-// gradient, every list sum) of layers with padded channel counts.  These layers ran on the CUDA cores before
-// they came here, with products and sums in float32; one part per value - what the layers with whole
-// 64-channel blocks have always had - would round each operand to 8 bits.  The weights, grad_output of the weight
-// gradient and nearest taps are bf16 as they are.
-static bool padded_channels(int c) { return c % 64 != 0; }
-static bool split_fwd(const mc_desc* d) { return padded_channels(d->C_out) && (d->interp == 1 || d->interp == 2); }
-static bool split_dgrad(const mc_desc* d) { return padded_channels(d->C_out) || padded_channels(d->C_in); }
-
 static bool gather_by_tma(const mc_desc* d, const void* x, const void* tab, CUtensorMap* tm) {
   return d->interp == 0 && d->C_in % 64 == 0 && tapmap_compact(d, tab) &&
          make_gather_map(tm, x, (long)d->B * d->IH * d->IW, d->C_in);
 }
 
+// map != null: the kernel decodes the map itself; tab != null: prebuilt table (tapmap_build_launch)
 static int fwd_launch_impl(const mc_desc* d, const void* x, const void* map, const void* tab,
                            const void* w, const void* bias, void* y, void* ws, size_t ws_bytes,
                            cudaStream_t st) {
@@ -2297,7 +2302,7 @@ bool conv_tc_dgrad_supported(const mc_desc* d) {
   // (channels in 16-byte pieces on both sides; an image with fewer than 8 channels would also leave nearly all
   // of the 64 output columns empty)
   if (d->C_out % 8 != 0 || d->C_in % 8 != 0 || (long)d->K * d->C_out >= (1L << 24)) return false;
-  if (!invmap_supported(d)) return false;
+  if (!invmap_supported(d) || (split_dgrad(d) && !indexable(d))) return false;
   GemmPlan p;
   return plan_gemm(pad64(d->C_in), dgrad_slices(d), d->K, p);
 }
@@ -2363,6 +2368,7 @@ static bool plan_wgrad(const mc_desc* d, size_t tabb, WgradPlan& p) {
 
 bool conv_tc_wgrad_supported(const mc_desc* d) {
   if (d->dtype != MC_BF16 || d->layout != MC_NHWC || d->P != 0) return false;
+  if (padded_channels(d->C_out) && !indexable(d)) return false;
   WgradPlan p;
   return plan_wgrad(d, tap_table_bytes(d->K), p);
 }

@@ -110,6 +110,41 @@ def test_fused_activation_keeps_nan(cout, weighted):
     assert torch.equal(want.nan_to_num(), got.nan_to_num())
 
 
+@pytest.mark.parametrize("shift,ws", [(0, False), (1, True), (1, False), (0, True)])
+def test_c_entry_points_without_workspace_or_alignment(shift, ws):
+    """Multiples of 8 that are not multiples of 64: any element-aligned pointer, workspace or not, same result up
+    to the order of the sums."""
+    import ctypes
+    from mappedconvolutions_b200 import _lib
+    L = _lib.lib()
+    x, gy, w, b, m, K, interp = _case(16, 40, 1, 5)
+    d = _lib.McDesc(2, 16, 40, 10, 13, 9, 17, K, 0, 1, _lib.MC_BF16, _lib.MC_NHWC)
+
+    def dev(t):  # channels-last, off a 16-byte boundary by `shift` elements
+        t = t.permute(0, 2, 3, 1).contiguous()
+        buf = torch.empty(t.numel() + 16, dtype=t.dtype, device="cuda")
+        out = buf[shift:shift + t.numel()].view(t.shape)
+        out.copy_(t)
+        return out
+
+    xd, gd, wd, bd, md = dev(x), dev(gy), w.cuda(), b.cuda(), m.cuda()
+    y = dev(torch.zeros(2, 40, 9, 17, dtype=torch.bfloat16))
+    gw, gb = torch.empty(40, 16, K, device="cuda"), torch.empty(40, device="cuda")
+    n = L.mc_conv_fwd_workspace_bytes(ctypes.byref(d))
+    buf = torch.empty(n, dtype=torch.uint8, device="cuda")
+    st = torch.cuda.current_stream().cuda_stream
+    _lib.check(L.mc_conv_fwd(ctypes.byref(d), xd.data_ptr(), md.data_ptr(), None, wd.data_ptr(), bd.data_ptr(), y.data_ptr(),
+                             buf.data_ptr() if ws else None, n if ws else 0, st))
+    _lib.check(L.mc_conv_wgrad(ctypes.byref(d), gd.data_ptr(), xd.data_ptr(), md.data_ptr(), None, gw.data_ptr(),
+                               gb.data_ptr(), None, 0, st))
+    f = [t.float() for t in (x, gy, w, b)]
+    want = oracle.mapped_conv_forward(f[0], m, f[2], f[3], K, 1)
+    _, want_gw, want_gb = oracle.mapped_conv_backward(f[1], m, f[0], f[2], f[3], K, 1)
+    H.assert_close(y.float().permute(0, 3, 1, 2), want, 2.0 ** -7, "y")  # (one rounding)
+    H.assert_close(gw, want_gw, 1e-4, "gw")  # (float32 sums of values that keep 16 bits)
+    H.assert_close(gb, want_gb, 1e-5, "gb")
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("B,C,H_,W_", [(1, 64, 8, 8), (3, 65, 7, 9), (2, 17, 1, 130), (2, 3, 5, 7), (1, 200, 3, 3), (5, 16, 1, 1),
                                        (1, 20, 64, 65)])
