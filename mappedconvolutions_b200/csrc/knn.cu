@@ -3,8 +3,8 @@
 //     points stream through shared memory in tiles that every thread of the block reads as a broadcast;
 //   * few queries: one or several warps per query, merged at the end;
 //   * many pairs, D <= 3: references and queries sorted along a Morton curve, 32 references to a leaf
-//     with its bounding box, and a warp of 32 neighbouring queries that only looks at leaves whose
-//     box can still hold one of the k nearest points.
+//     with its bounding box, and a warp per query that only looks at leaves whose box can still hold
+//     one of the k nearest points.
 // Semantics restated from the reference's include/util/cuda/knn.cuh:
 //   distance  :82-103   ssd over the dimensions in order, here pinned to s = fmaf(t, t, s) with
 //                       t = ref_i - query_i starting from s = 0
@@ -93,33 +93,144 @@ struct WarpTopK {
   }
 };
 
-// Launched behind the search among sorted leaves, the all-pairs kernels only run if that has given up:
-// `crowded` counts the leaves in crowded places, see knn_leaves_kernel.
-struct KnnGate {
-  const int* crowded;  // null: run
+// The queries of an all-pairs kernel.  On its own it takes all of them.  Behind the search among sorted leaves it
+// takes what the search has left: everything where the references are crowded (see knn_leaves_kernel), else the
+// queries that were listed (see knn_tree_kernel) - a warp or several per query where these are few.
+struct KnnTodo {
+  const int* crowded;  // leaves in crowded places; null: not behind a search
+  const int* count;    // [B] queries listed
+  const int* list;     // [B][N]
   int nleaf;           // leaves in all
-  __device__ __forceinline__ bool tree() const { return crowded && __ldg(crowded) <= nleaf / 8; }
+  int few;             // up to here: warps per query
+  __device__ __forceinline__ bool searched() const { return __ldg(crowded) <= nleaf / 8; }
+  // how many queries of batch b there are, and their list (null: 0, 1, ..)
+  __device__ __forceinline__ int take(int b, int N, const int** from) const {
+    *from = nullptr;
+    if (!crowded || !searched()) return N;
+    *from = list + (long)b * N;
+    return __ldg(count + b);
+  }
 };
 
 constexpr int KNN_THREADS = 256;
 constexpr int KNN_TILE = 512;
 constexpr int KNN_DMAX = 16;
+constexpr int KNNT_DMAX = 3;  // dimensions the search among sorted leaves takes
 
+// ---- few queries: a warp, or several, per query -----------------------------------------------------
+// One thread per query leaves the chip idle when there are few: 200 queries are two blocks of the kernels
+// below, whose threads walk 160 000 references one after another (2.9 ms).  Here the lanes of a warp look
+// at 32 references at a time (coalesced loads, four in flight per coordinate) for one query, whose list is
+// spread over the lanes; wpq warps share a query's references and the first one merges their lists.
+constexpr int KNNW_WARPS = 8;       // warps of a block that takes several queries
+constexpr int KNNW_MAX_WARPS = 32;  // warps that share one query at most
+
+// Enough warps for the chip, at least 16 references per lane.
+__host__ __device__ __forceinline__ int knn_warps_per_query(long queries, int M, int most) {
+  int wpq = 1;
+  while (wpq < most && queries * wpq < 148 * 16 && M >= 2 * wpq * 32 * 16) wpq *= 2;
+  return wpq;
+}
+
+__device__ __forceinline__ void knn_store(int64_t* idx, float* dist, long o, float d, int i) {
+  idx[o] = d == INFINITY ? 0 : (int64_t)i + 1;
+  dist[o] = __fsqrt_rn(d);
+}
+
+// Queries [0, total) of batch b (through `from`, if any), dealt out to the grid's blocks; sd, si: one row per warp.
+template <int DT>
+__device__ __forceinline__ void knn_wide(const float* __restrict__ ref, const float* __restrict__ query, int D, int M,
+                                         int N, int k, int64_t* __restrict__ idx, float* __restrict__ dist, int b,
+                                         const int* from, int total, float (*sd)[32], int (*si)[32]) {
+  constexpr int DS = DT > 0 ? DT : KNN_DMAX;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warps = blockDim.x >> 5, wpq = knn_warps_per_query((long)total * gridDim.y, M, warps), qpb = warps / wpq;
+  const int part = warp % wpq;
+  const float* rb = ref + (long)b * D * M;
+  const float* qb = query + (long)b * D * N;
+  for (int q0 = blockIdx.x * qpb; q0 < total; q0 += gridDim.x * qpb) {
+    const int slot = q0 + warp / wpq;
+    const bool live = slot < total;
+    const int n = live && from ? __ldg(from + slot) : slot;
+    WarpTopK top;
+    top.init();
+    if (live) {
+      float q[DS];
+#pragma unroll
+      for (int i = 0; i < DS; ++i) q[i] = i < D ? __ldg(qb + (long)i * N + n) : 0.f;
+      constexpr int U = 4;
+      bool first = true;
+      for (int m0 = part * 32; m0 < M; m0 += wpq * 32 * U) {
+        float s[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) s[u] = 0.f;
+#pragma unroll
+        for (int i = 0; i < DS; ++i) {
+          if (DT == 0 && i >= D) break;
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            const int j = m0 + u * wpq * 32 + lane;
+            const float t = (j < M ? __ldg(rb + (long)i * M + j) : INFINITY) - q[i];
+            s[u] = fmaf(t, t, s[u]);
+          }
+        }
+        int u0 = 0;
+        if (first) { top.fill(s[0], m0 + lane, k, lane); first = false; u0 = 1; }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+          if (u >= u0) top.offer<true>(s[u], m0 + u * wpq * 32 + lane, k, lane);
+      }
+    }
+    if (wpq > 1) {
+      sd[warp][lane] = top.d;
+      si[warp][lane] = top.i;
+      __syncthreads();
+      if (part == 0)
+        for (int p = 1; p < wpq; ++p)
+          top.offer<false>(lane < k ? sd[warp + p][lane] : INFINITY, si[warp + p][lane], k, lane);
+      __syncthreads();
+    }
+    if (part == 0 && live && lane < k) knn_store(idx, dist, ((long)b * k + lane) * N + n, top.d, top.i);
+  }
+}
+
+template <int DT>
+__global__ void __launch_bounds__(KNNW_MAX_WARPS * 32, 1) knn_wide_kernel(const float* __restrict__ ref,
+                                                                      const float* __restrict__ query, int D, int M,
+                                                                      int N, int k, int64_t* __restrict__ idx,
+                                                                      float* __restrict__ dist) {
+  __shared__ float sd[KNNW_MAX_WARPS][32];
+  __shared__ int si[KNNW_MAX_WARPS][32];
+  knn_wide<DT>(ref, query, D, M, N, k, idx, dist, blockIdx.y, nullptr, N, sd, si);
+}
+
+// ---- one thread per query ---------------------------------------------------------------------------
 // DT > 0: compile-time dimension; DT == 0: runtime dimension up to KNN_DMAX.
 template <int DT, int KMAX>
 __global__ void __launch_bounds__(KNN_THREADS) knn_kernel(const float* __restrict__ ref,
                                                           const float* __restrict__ query, int D,
                                                           int M, int N, int k,
                                                           int64_t* __restrict__ idx,
-                                                          float* __restrict__ dist, KnnGate gate) {
-  if (gate.tree()) return;
+                                                          float* __restrict__ dist, KnnTodo todo) {
   constexpr int DS = DT > 0 ? DT : KNN_DMAX;
   __shared__ float tile[DS][KNN_TILE];
   const int b = blockIdx.y;
   const float* rb = ref + (long)b * D * M;
   const float* qb = query + (long)b * D * N;
-  const int n = blockIdx.x * KNN_THREADS + threadIdx.x;
-  const bool live = n < N;
+  const int* from;
+  const int total = todo.take(b, N, &from);
+  if constexpr (DT > 0 && DT <= KNNT_DMAX) {
+    if (todo.crowded && total <= todo.few) {
+      __shared__ float sd[KNN_THREADS / 32][32];
+      __shared__ int si[KNN_THREADS / 32][32];
+      knn_wide<DT>(ref, query, D, M, N, k, idx, dist, b, from, total, sd, si);
+      return;
+    }
+  }
+  if (blockIdx.x * KNN_THREADS >= (unsigned)total) return;
+  const int slot = blockIdx.x * KNN_THREADS + threadIdx.x;
+  const bool live = slot < total;
+  const int n = live && from ? __ldg(from + slot) : slot;
   float q[DS];
 #pragma unroll
   for (int i = 0; i < DS; ++i) q[i] = (live && i < D) ? qb[(long)i * N + n] : 0.f;
@@ -184,14 +295,25 @@ __global__ void __launch_bounds__(KNN2_THREADS, KMAX <= 12 ? KNN2_BLOCKS_PER_SM 
                                                                    const float* __restrict__ query,
                                                                    int M, int N, int k,
                                                                    int64_t* __restrict__ idx,
-                                                                   float* __restrict__ dist, KnnGate gate) {
-  if (gate.tree()) return;
+                                                                   float* __restrict__ dist, KnnTodo todo) {
   __shared__ __align__(16) float tile[DT][KNN2_TILE];
   const int b = blockIdx.y;
   const float* rb = ref + (long)b * DT * M;
   const float* qb = query + (long)b * DT * N;
-  const int n = blockIdx.x * KNN2_THREADS + threadIdx.x;
-  const bool live = n < N;
+  const int* from;
+  const int total = todo.take(b, N, &from);
+  if constexpr (DT > 0 && DT <= KNNT_DMAX) {
+    if (todo.crowded && total <= todo.few) {
+      __shared__ float sd[KNN2_THREADS / 32][32];
+      __shared__ int si[KNN2_THREADS / 32][32];
+      knn_wide<DT>(ref, query, DT, M, N, k, idx, dist, b, from, total, sd, si);
+      return;
+    }
+  }
+  if (blockIdx.x * KNN2_THREADS >= (unsigned)total) return;
+  const int slot = blockIdx.x * KNN2_THREADS + threadIdx.x;
+  const bool live = slot < total;
+  const int n = live && from ? __ldg(from + slot) : slot;
   float2 nq[DT];  // (-q_i, -q_i)
 #pragma unroll
   for (int i = 0; i < DT; ++i) {
@@ -244,74 +366,6 @@ __global__ void __launch_bounds__(KNN2_THREADS, KMAX <= 12 ? KNN2_BLOCKS_PER_SM 
 }
 
 
-// ---- few queries: a warp, or several, per query -----------------------------------------------------
-// One thread per query leaves the chip idle when there are few: 200 queries are two blocks of the kernel
-// above, whose threads walk 160 000 references one after another (2.9 ms).  Here the lanes of a warp look
-// at 32 references at a time (coalesced loads, four in flight per coordinate) for one query, whose list is
-// spread over the lanes; wpq warps share a query's references and the first one merges their lists.
-constexpr int KNNW_WARPS = 8;       // warps of a block that takes several queries
-constexpr int KNNW_MAX_WARPS = 32;  // warps that share one query at most
-
-__device__ __forceinline__ void knn_store(int64_t* idx, float* dist, long o, float d, int i) {
-  idx[o] = d == INFINITY ? 0 : (int64_t)i + 1;
-  dist[o] = __fsqrt_rn(d);
-}
-
-template <int DT>
-__global__ void __launch_bounds__(KNNW_MAX_WARPS * 32) knn_wide_kernel(const float* __restrict__ ref,
-                                                                   const float* __restrict__ query, int D,
-                                                                   int M, int N, int k, int wpq,
-                                                                   int64_t* __restrict__ idx,
-                                                                   float* __restrict__ dist, KnnGate gate) {
-  if (gate.tree()) return;
-  constexpr int DS = DT > 0 ? DT : KNN_DMAX;
-  __shared__ float sd[KNNW_MAX_WARPS][32];
-  __shared__ int si[KNNW_MAX_WARPS][32];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int b = blockIdx.y;
-  const int n = blockIdx.x * (blockDim.x / 32 / wpq) + warp / wpq, part = warp % wpq;
-  const float* rb = ref + (long)b * D * M;
-  const float* qb = query + (long)b * D * N;
-  WarpTopK top;
-  top.init();
-  if (n < N) {
-    float q[DS];
-#pragma unroll
-    for (int i = 0; i < DS; ++i) q[i] = i < D ? __ldg(qb + (long)i * N + n) : 0.f;
-    constexpr int U = 4;
-    bool first = true;
-    for (int m0 = part * 32; m0 < M; m0 += wpq * 32 * U) {
-      float s[U];
-#pragma unroll
-      for (int u = 0; u < U; ++u) s[u] = 0.f;
-#pragma unroll
-      for (int i = 0; i < DS; ++i) {
-        if (DT == 0 && i >= D) break;
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-          const int j = m0 + u * wpq * 32 + lane;
-          const float t = (j < M ? __ldg(rb + (long)i * M + j) : INFINITY) - q[i];
-          s[u] = fmaf(t, t, s[u]);
-        }
-      }
-      int u0 = 0;
-      if (first) { top.fill(s[0], m0 + lane, k, lane); first = false; u0 = 1; }
-#pragma unroll
-      for (int u = 0; u < U; ++u)
-        if (u >= u0) top.offer<true>(s[u], m0 + u * wpq * 32 + lane, k, lane);
-    }
-  }
-  if (wpq > 1) {
-    sd[warp][lane] = top.d;
-    si[warp][lane] = top.i;
-    __syncthreads();
-    if (part == 0)
-      for (int p = 1; p < wpq; ++p)
-        top.offer<false>(lane < k ? sd[warp + p][lane] : INFINITY, si[warp + p][lane], k, lane);
-  }
-  if (part == 0 && n < N && lane < k) knn_store(idx, dist, ((long)b * k + lane) * N + n, top.d, top.i);
-}
-
 // ---- many pairs: leaves on a Morton curve -----------------------------------------------------------
 // 163 842 x 163 842 points are 2.7e10 pairs: 7.6 ms at the rate of the packed arithmetic above, while
 // all but about a hundred references per query can be ruled out by their position.  Keys of all
@@ -327,6 +381,12 @@ __global__ void __launch_bounds__(KNNW_MAX_WARPS * 32) knn_wide_kernel(const flo
 // in the box, and "skip if box distance > k-th distance" cannot lose a point, ties included (equal
 // distances are ordered by index, hence no skip at equality).
 // NaN references are outside every box and never nearer than anything.
+// What a box rules out depends on the queries too: one in the middle of a sphere of references, or far from all of
+// them, is about as far from every leaf and would visit them all, 32 points at a time, at up to four times the
+// cost of all pairs.  A query that has visited a quarter of the leaves is therefore given up and listed for the
+// all-pairs kernels, and once a thirty-second of a batch's queries is listed, others that have visited 64 leaves
+// follow.  163 842 references on the sphere and as many queries at its centre 34.1 -> 9.9 ms (all pairs: 8.4 ms), 160 000
+// and 2 000 1.59 -> 1.02 ms; queries on the sphere 312 -> 323 us.
 // (Tried first: one query per lane and 32 neighbouring queries per warp, every lane testing the points of
 // all leaves that one of them needs: 271 us for the search alone, and far slower than all pairs where
 // queries are sparse among the references.)
@@ -517,8 +577,9 @@ __global__ void __launch_bounds__(KNNT_WARPS * 32) knn_tree_kernel(
     const float* __restrict__ query, int M, int N, int k, int nleaf, int nnode, int ngroup,
     const unsigned* __restrict__ keys, const unsigned* __restrict__ qkeys, const int* __restrict__ qvals,
     const float* __restrict__ leaves, const float* __restrict__ lbox, const float* __restrict__ nbox,
-    const float* __restrict__ gbox, KnnGate gate, int64_t* __restrict__ idx, float* __restrict__ dist) {
-  if (!gate.tree()) return;
+    const float* __restrict__ gbox, KnnTodo todo, int* __restrict__ listed, int* __restrict__ list, int budget,
+    int64_t* __restrict__ idx, float* __restrict__ dist) {
+  if (!todo.searched()) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int b = blockIdx.y;
   constexpr int LSTRIDE = (DT + 1) * KNNT_LEAF, BSTRIDE = 2 * DT * 32;
@@ -572,6 +633,7 @@ __global__ void __launch_bounds__(KNNT_WARPS * 32) knn_tree_kernel(
   bool nan = false;
 #pragma unroll
   for (int i = 0; i < DT; ++i) nan |= q[i] != q[i];
+  int seen = 0;  // leaves visited
   for (int g0 = 0; g0 < ngroup && !nan; g0 += 32) {
     float ggap = box_gap2<DT>(q, gb + (g0 / 32) * BSTRIDE);
     for (int gs; (gs = pop_nearest(ggap, top.thr, lane)) >= 0;) {
@@ -585,14 +647,25 @@ __global__ void __launch_bounds__(KNNT_WARPS * 32) knn_tree_kernel(
           point(l0 + ls, s, j);
           top.offer<false>(s, j, k, lane);
         }
+        // (added up per node: a counter in the loop over leaves makes the search 8 % slower)
+        seen += __popc(__ballot_sync(0xffffffffu, lgap == INFINITY));
+        if (seen > 64) {
+          int others = lane == 0 ? *(volatile const int*)(listed + b) : 0;
+          others = __shfl_sync(0xffffffffu, others, 0);
+          if (seen > budget || others > N / 32) top.thr = -1.f;  // (no box passes any more)
+        }
       }
     }
+  }
+  if (top.thr < 0.f) {
+    if (lane == 0) list[(long)b * N + atomicAdd(listed + b, 1)] = n;
+    return;
   }
   if (lane < k) knn_store(idx, dist, ((long)b * k + lane) * N + n, top.d, top.i);
 }
 
 struct KnnTreeWs {
-  size_t bounds, keys_in, keys, vals_in, vals, leaves, lbox, nbox, gbox, cub, cub_bytes, total;
+  size_t list, bounds, keys_in, keys, vals_in, vals, leaves, lbox, nbox, gbox, cub, cub_bytes, total;
   long items;
   int nleaf, nnode, ngroup, end_bit;
 };
@@ -607,7 +680,8 @@ static KnnTreeWs knn_tree_layout(int B, int D, int M, int N, bool same) {
   while ((1L << (L.end_bit - KNNT_BITS)) < (same ? B : 2L * B)) ++L.end_bit;
   size_t o = 0;
   auto take = [&](size_t n) { const size_t at = o; o += (n + 255) & ~(size_t)255; return at; };
-  L.bounds = take((size_t)B * 2 * D * 4 + 16);  // (and the count of crowded leaves)
+  L.bounds = take((size_t)B * (2 * D + 1) * 4 + 16);  // (and the counts of listed queries and crowded leaves)
+  L.list = take((size_t)B * N * 4);
   L.keys_in = take((size_t)L.items * 4);
   L.keys = take((size_t)L.items * 4);
   L.vals_in = take((size_t)L.items * 4);
@@ -625,8 +699,9 @@ static KnnTreeWs knn_tree_layout(int B, int D, int M, int N, bool same) {
 }
 
 template <int DT>
-static void knn_brute_launch(const float* ref, const float* query, int B, int D, int M, int N, int k,
-                             int64_t* idx, float* dist, cudaStream_t st, KnnGate gate = {nullptr, 0});
+static void knn_thread_launch(const float* ref, const float* query, int B, int D, int M, int N, int k,
+                              int64_t* idx, float* dist, cudaStream_t st, const KnnTodo& todo);
+static long knn_few(int D, int M);
 
 template <int DT>
 static int knn_tree_launch(const float* ref, const float* query, int B, int M, int N, int k, int64_t* idx,
@@ -640,8 +715,10 @@ static int knn_tree_launch(const float* ref, const float* query, int B, int M, i
   int *vals_in = (int*)(p + L.vals_in), *vals = (int*)(p + L.vals);
   float *leaves = (float*)(p + L.leaves), *lbox = (float*)(p + L.lbox), *nbox = (float*)(p + L.nbox),
         *gbox = (float*)(p + L.gbox);
-  int* crowded = (int*)(bounds + (long)B * 2 * DT);
-  if (cudaMemsetAsync(bounds, 0, (size_t)B * 2 * DT * 4 + 4, st) != cudaSuccess) return MC_ERR_LAUNCH;
+  int* listed = (int*)(bounds + (long)B * 2 * DT);
+  int* crowded = listed + B;
+  int* list = (int*)(p + L.list);
+  if (cudaMemsetAsync(bounds, 0, (size_t)B * (2 * DT + 1) * 4 + 4, st) != cudaSuccess) return MC_ERR_LAUNCH;
   int bb = (M + 1023) / 1024;
   if (bb > 148) bb = 148;
   knn_bounds_kernel<DT><<<dim3(bb, B), 256, 0, st>>>(ref, M, bounds), MC_COUNT(1);
@@ -654,15 +731,17 @@ static int knn_tree_launch(const float* ref, const float* query, int B, int M, i
   knn_leaves_kernel<DT><<<dim3(L.nnode, B), 1024, 0, st>>>(ref, M, L.nleaf, keys, vals, leaves, lbox, nbox, L.ngroup,
                                                            crowded), MC_COUNT(1);
   knn_groups_kernel<DT><<<dim3((L.ngroup + 31) / 32 * 32, B), 32, 0, st>>>(nbox, L.nnode, L.ngroup, gbox), MC_COUNT(1);
-  const KnnGate gate = {crowded, L.nleaf * B};
+  const KnnTodo todo = {crowded, listed, list, L.nleaf * B, (int)(knn_few(DT, M) / B)};
+  const int budget = L.nleaf / 4 > 128 ? L.nleaf / 4 : 128;
   const unsigned* qkeys = same ? nullptr : keys + (long)B * M;
   const int* qvals = same ? vals : vals + (long)B * M;
   // one query per warp: queries cost between one and several times the average, and a warp (or a block) that
   // takes several of them makes the last wave longer (8 per warp: 298 us instead of 232 us at 163 842 x 163 842)
   const dim3 grid((unsigned)((N + KNNT_WARPS - 1) / KNNT_WARPS), (unsigned)B);
   knn_tree_kernel<DT><<<grid, KNNT_WARPS * 32, 0, st>>>(query, M, N, k, L.nleaf, L.nnode, L.ngroup, keys,
-                                                        qkeys, qvals, leaves, lbox, nbox, gbox, gate, idx, dist), MC_COUNT(1);
-  knn_brute_launch<DT>(ref, query, B, DT, M, N, k, idx, dist, st, gate);
+                                                        qkeys, qvals, leaves, lbox, nbox, gbox, todo, listed, list,
+                                                        budget, idx, dist), MC_COUNT(1);
+  knn_thread_launch<DT>(ref, query, B, DT, M, N, k, idx, dist, st, todo);
   MC_CHECK_LAUNCH();
   return MC_OK;
 }
@@ -671,31 +750,42 @@ static int knn_tree_launch(const float* ref, const float* query, int B, int M, i
 // a warp per query needs about 1.5 ps per pair + 1 ns per query (a reference is loaded again for every
 // query), which is less up to some 20 000 queries.
 constexpr long KNN_WIDE_QUERIES = 20000;
+static long knn_few(int, int) { return KNN_WIDE_QUERIES; }
+
+// one thread per query; behind the search as many blocks as the chip holds, for the case of a warp per query
+static int knn_blocks(int N, int threads, const KnnTodo& todo) {
+  const int n = (N + threads - 1) / threads;
+  return todo.crowded && n < 148 * 8 ? 148 * 8 : n;
+}
+template <int DT>
+static void knn_thread_launch(const float* ref, const float* query, int B, int D, int M, int N, int k,
+                              int64_t* idx, float* dist, cudaStream_t st, const KnnTodo& todo) {
+  if (DT > 0 && k <= 16) {
+    constexpr int DS = DT > 0 ? DT : 1;
+    dim3 grid((unsigned)knn_blocks(N, KNN2_THREADS, todo), (unsigned)B);
+    if (k <= 8) knn_small_d_kernel<DS, 8><<<grid, KNN2_THREADS, 0, st>>>(ref, query, M, N, k, idx, dist, todo), MC_COUNT(1);
+    else if (k <= 12) knn_small_d_kernel<DS, 12><<<grid, KNN2_THREADS, 0, st>>>(ref, query, M, N, k, idx, dist, todo), MC_COUNT(1);
+    else knn_small_d_kernel<DS, 16><<<grid, KNN2_THREADS, 0, st>>>(ref, query, M, N, k, idx, dist, todo), MC_COUNT(1);
+    return;
+  }
+  dim3 grid((unsigned)knn_blocks(N, KNN_THREADS, todo), (unsigned)B);
+  if (k <= 8) knn_kernel<DT, 8><<<grid, KNN_THREADS, 0, st>>>(ref, query, D, M, N, k, idx, dist, todo), MC_COUNT(1);
+  else if (k <= 16) knn_kernel<DT, 16><<<grid, KNN_THREADS, 0, st>>>(ref, query, D, M, N, k, idx, dist, todo), MC_COUNT(1);
+  else knn_kernel<DT, 32><<<grid, KNN_THREADS, 0, st>>>(ref, query, D, M, N, k, idx, dist, todo), MC_COUNT(1);
+}
 
 template <int DT>
 static void knn_brute_launch(const float* ref, const float* query, int B, int D, int M, int N, int k,
-                             int64_t* idx, float* dist, cudaStream_t st, KnnGate gate) {
+                             int64_t* idx, float* dist, cudaStream_t st) {
   const long queries = (long)B * N;
-  if (queries <= KNN_WIDE_QUERIES) {
-    int wpq = 1;  // enough warps for the chip, at least 16 references per lane
-    while (wpq < KNNW_MAX_WARPS && queries * wpq < 148 * 16 && M >= 2 * wpq * 32 * 16) wpq *= 2;
-    const int warps = wpq > KNNW_WARPS ? wpq : KNNW_WARPS, qpb = warps / wpq;
-    knn_wide_kernel<DT><<<dim3((unsigned)((N + qpb - 1) / qpb), (unsigned)B), warps * 32, 0, st>>>(
-        ref, query, D, M, N, k, wpq, idx, dist, gate), MC_COUNT(1);
+  if (queries > knn_few(D, M)) {
+    knn_thread_launch<DT>(ref, query, B, D, M, N, k, idx, dist, st, KnnTodo{});
     return;
   }
-  if (DT > 0 && k <= 16) {
-    constexpr int DS = DT > 0 ? DT : 1;
-    dim3 grid((unsigned)((N + KNN2_THREADS - 1) / KNN2_THREADS), (unsigned)B);
-    if (k <= 8) knn_small_d_kernel<DS, 8><<<grid, KNN2_THREADS, 0, st>>>(ref, query, M, N, k, idx, dist, gate), MC_COUNT(1);
-    else if (k <= 12) knn_small_d_kernel<DS, 12><<<grid, KNN2_THREADS, 0, st>>>(ref, query, M, N, k, idx, dist, gate), MC_COUNT(1);
-    else knn_small_d_kernel<DS, 16><<<grid, KNN2_THREADS, 0, st>>>(ref, query, M, N, k, idx, dist, gate), MC_COUNT(1);
-    return;
-  }
-  dim3 grid((unsigned)((N + KNN_THREADS - 1) / KNN_THREADS), (unsigned)B);
-  if (k <= 8) knn_kernel<DT, 8><<<grid, KNN_THREADS, 0, st>>>(ref, query, D, M, N, k, idx, dist, gate), MC_COUNT(1);
-  else if (k <= 16) knn_kernel<DT, 16><<<grid, KNN_THREADS, 0, st>>>(ref, query, D, M, N, k, idx, dist, gate), MC_COUNT(1);
-  else knn_kernel<DT, 32><<<grid, KNN_THREADS, 0, st>>>(ref, query, D, M, N, k, idx, dist, gate), MC_COUNT(1);
+  const int wpq = knn_warps_per_query(queries, M, KNNW_MAX_WARPS);
+  const int warps = wpq > KNNW_WARPS ? wpq : KNNW_WARPS, qpb = warps / wpq;
+  knn_wide_kernel<DT><<<dim3((unsigned)((N + qpb - 1) / qpb), (unsigned)B), warps * 32, 0, st>>>(
+      ref, query, D, M, N, k, idx, dist), MC_COUNT(1);
 }
 
 static int knn_check(const void* ref, const void* query, int B, int D, int M, int N, int k, const void* idx,
@@ -708,7 +798,7 @@ static int knn_check(const void* ref, const void* query, int B, int D, int M, in
 }
 
 static bool knn_tree_shape(int B, int D, int M, int N) {
-  return D <= 3 && B <= 128 && (long)B * ((long)M + N) < (1L << 30);
+  return D <= KNNT_DMAX && B <= 128 && (long)B * ((long)M + N) < (1L << 30);
 }
 
 }  // namespace mc

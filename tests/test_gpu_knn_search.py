@@ -59,3 +59,24 @@ def test_knn_of_a_set_with_itself():
     idx, dist = host.impl.knn_forward(d, d, 9)
     want_idx, want_dist = oracle.knn_forward(p, p, 9)
     assert torch.equal(idx.cpu(), want_idx) and torch.equal(dist.cpu(), want_dist)
+
+
+# Queries that no box rules anything out for: at the centre of a sphere of references, or far away from all; all of
+# them, some of them (listed for the all-pairs kernels one by one), in one batch element of two
+@pytest.mark.parametrize("B,D,M,N,k,share", [(1, 3, 70001, 900, 9, 1.0), (1, 3, 9001, 7001, 9, 1.0), (1, 3, 40000, 30000, 5, 0.8),
+                                             (1, 3, 40000, 2000, 20, 0.02), (2, 2, 20000, 3000, 9, 0.5),
+                                             (1, 1, 40000, 1300, 3, 0.5)])
+def test_queries_at_the_same_distance_from_everything(B, D, M, N, k, share):
+    from mappedconvolutions_b200 import host
+    g = torch.Generator().manual_seed(M)
+    ref, query = _points("sphere", B, D, M, g), _points("sphere", B, D, N, g)
+    if D == 1:
+        ref = torch.randn(B, D, M, generator=g)
+    n = int(share * N)
+    where = torch.randperm(N, generator=g)[:n]
+    query[0, :, where[::2]] *= 1e-3
+    query[0, :, where[1::2]] *= 1e4
+    idx, dist = host.impl.knn_forward(ref.cuda(), query.cuda(), k)
+    want_idx, want_dist = oracle.knn_forward(ref, query, k)
+    assert torch.equal(idx.cpu(), want_idx)
+    assert torch.equal(dist.cpu(), want_dist)
