@@ -746,11 +746,18 @@ static int knn_tree_launch(const float* ref, const float* query, int B, int M, i
   return MC_OK;
 }
 
-// All pairs.  A thread per query needs about 40 us + 0.02 us per reference however few queries there are;
-// a warp per query needs about 1.5 ps per pair + 1 ns per query (a reference is loaded again for every
-// query), which is less up to some 20 000 queries.
-constexpr long KNN_WIDE_QUERIES = 20000;
-static long knn_few(int, int) { return KNN_WIDE_QUERIES; }
+// All pairs: up to how many queries a warp per query is the better choice.  It takes time for every pair, since each
+// query loads the references again; a thread per query takes the same time for any number of queries that the chip
+// holds.  Measured, in microseconds, warps / threads:
+//   D = 3, 20 000 references:  16 000 queries 494 / 582, 30 000 896 / 669;  160 000: 12 000 2984 / 3167, 16 000 3753 / 3167
+//   D = 4, 20 000 references:  20 000 queries 689 / 693;                    160 000:  8 000 2219 / 3312, 12 000 3374 / 3308
+//   D = 8,  2 000 references:  20 000 queries 208 / 269, 30 000 312 / 269;  160 000: 12 000 9234 / 11280, 16 000 11659 / 11282
+//   D = 16, 2 000 references:   8 000 queries 210 / 261, 12 000 320 / 263;  160 000:  2 000 5018 / 11420,  5 000 13843 / 11431
+static long knn_few(int D, int M) {
+  const double pair = D <= 4 ? 1.05e-3 + 0.15e-3 * D : D <= 8 ? 0.57e-3 * D : 0.95e-3 * D;  // ns
+  const double threads = D <= 4 ? 150e3 + 20. * M : 130e3 + 70. * M;                        // ns
+  return (long)(threads / (1.9 + pair * M));
+}
 
 // one thread per query; behind the search as many blocks as the chip holds, for the case of a warp per query
 static int knn_blocks(int N, int threads, const KnnTodo& todo) {
