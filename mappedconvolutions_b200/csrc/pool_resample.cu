@@ -117,11 +117,9 @@ __device__ __forceinline__ void scatter_tap(CT* plane, long sp, const MT* m, con
   }
 }
 
-// Scatter of `units` whole planes (NCHW) or images (NHWC) starting at unit u0; zero[0 .. nzero) is cleared on
-// the way (the next chunk's target).  OP_GATHER here means "adjoint of gather" (resample scatter, K = 1).
+// Scatter of `units` whole planes (NCHW) or images (NHWC) from unit u0 on, into a.out.  OP_GATHER here means "adjoint of gather" (resample scatter, K = 1).
 template <typename T, int OP>
-__global__ void __launch_bounds__(256) sample_bwd_kernel(ScatterArgs a, long u0, long units,
-                                                         typename Traits<T>::CT* zero, long nzero) {
+__global__ void __launch_bounds__(256) sample_bwd_kernel(ScatterArgs a, long u0, long units) {
   typedef typename Traits<T>::CT CT;
   typedef typename Traits<T>::MT MT;
   const T* g = (const T*)a.g;
@@ -134,7 +132,6 @@ __global__ void __launch_bounds__(256) sample_bwd_kernel(ScatterArgs a, long u0,
   const int pp = a.P > 0 ? a.P : 1;
   const long nt = (long)gridDim.x * 256;
   const long t0 = blockIdx.x * 256L + threadIdx.x;
-  for (long i = blockIdx.y * nt + t0; i < nzero; i += nt * gridDim.y) zero[i] = CT(0);
   for (long u = blockIdx.y; u < units; u += gridDim.y) {
     CT* img = (CT*)a.out + u * nimg;
     const long base = (u0 + u) * n;
@@ -244,33 +241,37 @@ static int launch_fwd(const mc_desc* d, const void* x, const void* map, const vo
   return MC_OK;
 }
 
-// The image side is zeroed and scattered into in chunks of whole planes / images that stay in L2: over the
-// whole tensor at once every atomic read-modify-write would fetch a line that the memset had already pushed out
-// to HBM.  Each launch clears the target of the next one.  bf16: the sums of a chunk are rounded into the result
-// before the next chunk reuses their buffer.  Max pooling and unpooling of 32 x 128 planes of 163 842 vertices: 3.47 ms
-// with one memset and one scatter, 3.14 ms in chunks of 32 MB (16 MB: 3.45, 64 MB: 3.97); what is left of the scatter
-// (1.85 of 2.18 ms) is the rate of scattered atomics in L2, about 86 per ns.
-constexpr long SCATTER_CHUNK_BYTES = 32L << 20;
+// float32 and float64: one memset and one scatter of everything.  (In chunks of whole planes that stay in L2, each
+// launch clearing the next one's target, every size is slower - max unpooling, everything / chunks of 64 / 32 / 16 MB:
+// 32 x 128 planes of 163 842 vertices 1539 / 1893 / 1972 / 2175 us, of 40 962 401 / 473 / 490 / 507 us, 8 x 64 planes
+// of 512 x 1024 pixels 840 / 943 / 915 / 922 us.)
+// bf16: the float32 sums of a chunk are rounded into the result before the next chunk reuses their buffer, so that they
+// stay in L2, with a third of it for them.  Max unpooling of bf16 in chunks of 24 / 32 / 43 / 64 / 96 MB: channels-last
+// 32 x 128 x 40 962 vertices 685 / 684 / 556 / 660 / 719 us, 32 x 256 x 10 242 364 / 318 / 290 / 335 / 364 us; planes, 32 x 64 x
+// 163 842 1386 / 1259 / 1214 / 1393 / 1496 us, 8 x 64 x 512 x 1024 1174 / 1065 / 1092 / 1268 / 1364 us.
+constexpr long SCATTER_CHUNK_BYTES = 42L << 20;
+
+// units: planes (NCHW) or images (NHWC) of unit_bytes
+static long scatter_units_per_chunk(long units, long unit_bytes) {
+  const long per = SCATTER_CHUNK_BYTES / unit_bytes;
+  return per < 1 ? 1 : per > units ? units : per;
+}
 
 template <typename T, int OP>
-static int launch_bwd_chunks(ScatterArgs a, typename Traits<T>::CT* acc, bf16* rounded, cudaStream_t st) {
+static int launch_bwd_units(ScatterArgs a, typename Traits<T>::CT* acc, bf16* rounded, cudaStream_t st) {
   typedef typename Traits<T>::CT CT;
   const bool nhwc = a.layout == MC_NHWC;
   const long nimg = nhwc ? a.npix_img * a.C : a.npix_img, n = nhwc ? a.npix_grid * a.C : a.npix_grid;
   const long units = nhwc ? a.B : (long)a.B * a.C;
-  long per = SCATTER_CHUNK_BYTES / (nimg * (long)sizeof(CT));
-  if (per < 1) per = 1;
-  if (per > units) per = units;
+  const long per = rounded ? scatter_units_per_chunk(units, nimg * (long)sizeof(CT)) : units;
+  a.out = acc;
   if (cudaMemsetAsync(acc, 0, per * nimg * sizeof(CT), st) != cudaSuccess) return MC_ERR_LAUNCH;
   const long vals = 256L * (OP == OP_MAX ? 4 : 1);
   const unsigned gx = (unsigned)((n + vals - 1) / vals < 148 * 32 ? (n + vals - 1) / vals : 148 * 32);
   for (long u0 = 0; u0 < units; u0 += per) {
     const long m = units - u0 < per ? units - u0 : per;
-    const long next = rounded ? 0 : (units - u0 - m < per ? units - u0 - m : per);
-    a.out = rounded ? acc : acc + u0 * nimg;
     const dim3 grid(gx, (unsigned)(m < 65535 ? m : 65535));
-    sample_bwd_kernel<T, OP><<<grid, 256, 0, st>>>(a, u0, m, rounded ? nullptr : acc + (u0 + m) * nimg,
-                                                   next * nimg), MC_COUNT(1);
+    sample_bwd_kernel<T, OP><<<grid, 256, 0, st>>>(a, u0, m), MC_COUNT(1);
     MC_CHECK_LAUNCH();
     if (rounded) {
       take_from_f32_kernel<bf16><<<grid_for(m * nimg, 256), 256, 0, st>>>((float*)acc, rounded + u0 * nimg,
@@ -292,10 +293,10 @@ static int launch_bwd(const mc_desc* d, const void* g, const int64_t* idx, const
   a.npix_grid = (long)d->OH * d->OW;
   if (OP == OP_GATHER && weighted3_ok(d))
     return weighted3_scatter_launch(d, (const float*)g, (const float*)map, (const float*)iw, (float*)out, st);
-  if (d->dtype == MC_F32) return launch_bwd_chunks<float, OP>(a, (float*)out, nullptr, st);
-  if (d->dtype == MC_F64) return launch_bwd_chunks<double, OP>(a, (double*)out, nullptr, st);
-  if (!ws || ws_bytes < (size_t)a.B * a.C * a.npix_img * sizeof(float)) return MC_ERR_WORKSPACE;
-  return launch_bwd_chunks<bf16, OP>(a, (float*)ws, (bf16*)out, st);
+  if (d->dtype == MC_F32) return launch_bwd_units<float, OP>(a, (float*)out, nullptr, st);
+  if (d->dtype == MC_F64) return launch_bwd_units<double, OP>(a, (double*)out, nullptr, st);
+  if (!ws || ws_bytes < mc_scatter_workspace_bytes(d)) return MC_ERR_WORKSPACE;
+  return launch_bwd_units<bf16, OP>(a, (float*)ws, (bf16*)out, st);
 }
 
 }  // namespace mc
@@ -305,8 +306,10 @@ using namespace mc;
 extern "C" {
 
 size_t mc_scatter_workspace_bytes(const mc_desc* d) {
-  if (!d || d->dtype != MC_BF16) return 0;
-  return (size_t)d->B * d->C_in * d->IH * d->IW * sizeof(float);
+  if (!d || d->dtype != MC_BF16 || d->B <= 0 || d->C_in <= 0 || d->IH <= 0 || d->IW <= 0) return 0;
+  const bool nhwc = d->layout == MC_NHWC;  // one chunk of float32 sums
+  const long unit = (long)d->IH * d->IW * (nhwc ? d->C_in : 1) * (long)sizeof(float);
+  return (size_t)(scatter_units_per_chunk(nhwc ? d->B : (long)d->B * d->C_in, unit) * unit);
 }
 
 int mc_pool_max_fwd(const mc_desc* d, const void* x, const void* map, const void* iw, void* y,
