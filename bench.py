@@ -614,7 +614,8 @@ def secondary_record(wl, steps, warmup, no_cpu, min_seconds=0.0):
     scale = 1e9
     ach = fam[top][1] / (times[top] * 1e-3) / scale
     if wl == "knn":
-        roof = {"bound": "fp32 CUDA cores (no HBM or tensor roofline applies)", "kernel": top,
+        # (pairs are counted as queries x references; the search among sorted leaves forms a small part of them)
+        roof = {"bound": "leaf visits of the search (L1 and issue; no HBM or tensor roofline applies)", "kernel": top,
                 "achieved": ach, "unit": unit, "peak": None, "frac": None, "traffic": None,
                 "ms_per_launch": {k: round(v, 4) for k, v in times.items()}}
     else:
